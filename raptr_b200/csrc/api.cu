@@ -360,7 +360,7 @@ struct Builder {
     int64_t per = std::max<int64_t>(1, int64_t(kStagingBudget / (size_t(H) * 8)));
     per = std::min<int64_t>(per, 65536);
     if (!ctx->h_pin) RCU(cudaMallocHost(&ctx->h_pin, 16 * sizeof(int64_t)));
-    // words 0-1: the dense kernel's flags, 2-3: the table kernel's (per buffer)
+    // words 0-1: the slab kernel's flags, 2-3: the table kernel's (per buffer)
     volatile int32_t* h_flags = reinterpret_cast<volatile int32_t*>(ctx->h_pin);
     volatile int64_t* h_total = ctx->h_pin + 2;
     cudaStream_t P = nullptr, S2 = nullptr;
@@ -459,9 +459,9 @@ struct Builder {
         }
         e = cudaStreamWaitEvent(P, ev_k[b], 0);
         if (!d_rays) {
-          // The rows the dense kernel left to the hash table, on the
+          // The rows the slab kernel left to the hash table, on the
           // placement stream: a row or two per chunk, which would otherwise
-          // hold up the next chunk's dense rows on the caller's stream.
+          // hold up the next chunk's slab rows on the caller's stream.
           if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_flags + 2 + b, 0, sizeof(int32_t), P);
           if (e == cudaSuccess)
             e = launch_sm_rows(level, ctx->dg, ctx->d_sincos, d_cnl, r, k, nrays, seed, nullptr, st_col[b],

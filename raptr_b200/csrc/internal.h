@@ -55,10 +55,10 @@ int sm_pick_level(const DGeom& g, int nrays);
 // Builds rows [row0, row0+nrows) of the list into staging slots (slot i at
 // st_col/st_val + i*capacity).  row_nnz[i] = entries, or -1 if the table
 // overflowed.  *d_flags |= 1 on overflow, |= 4 for a channel id out of range.
-// With d_table_reasons (4 ints) the rows the dense kernel leaves to the hash
+// With d_table_reasons (4 ints) the rows the slab kernel leaves to the hash
 // table are counted by reason: no slab axis, windows over the slot limit,
 // a ray outside the windows, a slot decoding outside the grid.  parts: 1 =
-// the dense kernel only (rows it cannot take keep row_nnz = -2), 2 = the
+// the slab kernel only (rows it cannot take keep row_nnz = -2), 2 = the
 // table kernel for those rows only, 3 = both; with d_rays every row takes
 // the table kernel whatever parts says.
 constexpr int kRowsDense = 1, kRowsTable = 2, kRowsAll = 3;

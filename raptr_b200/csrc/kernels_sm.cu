@@ -4,22 +4,20 @@
 // Row build (one CTA per channel row):
 //   1. thread 0 builds the channel state (both crystal transforms from the
 //      per-angle sine/cosine table, crystal centres, cylinder radius);
-//   2. every thread generates rays r = tid, tid+T, ... (Philox keyed by
-//      (seed, channel)) and walks each through the grid.  The walk visits
-//      exactly the voxels whose intersection length with the ray is positive
-//      and computes that length with the same float operations as the
-//      reference's intersectionLength (src/getSystemMatrixDeviceOnly.cu:129-174):
+//   2. the row's rays (Philox keyed by (seed, channel)) are traced through the
+//      grid.  A trace yields exactly the voxels whose intersection length with
+//      the ray is positive, and that length with the same float operations as
+//      the reference's intersectionLength (src/getSystemMatrixDeviceOnly.cu:129-174):
 //      per-axis plane parameters (face - start)/(end - start), masked max of
 //      the entry parameters, masked min of the exit parameters, and
-//      (exit - entry) * |end - start|.  Lengths are summed in shared memory:
-//      into dense per-slab windows of the voxels the row's rays can reach
-//      when the two crystals lie on opposite sides of the grid along x or z,
-//      else into an open-addressing hash table keyed by voxel id;
+//      (exit - entry) * |end - start|.  When the two crystals lie on opposite
+//      sides of the grid along x or z, threads own slabs of the grid
+//      (sm_slab_kernel); the other rows walk each ray from plane to plane into
+//      an open-addressing hash table keyed by voxel id (sm_table_kernel);
 //   3. the sums are compacted keeping voxels that pass the exact cylinder
 //      test (the reference only evaluates candidates,
-//      src/getSystemMatrixDeviceOnly.cu:433-470), put in voxel-id order
-//      (x-slab windows already are; the others are bitonic-sorted), divided
-//      by the ray count and written to the row's staging slot.
+//      src/getSystemMatrixDeviceOnly.cu:433-470), put in voxel-id order,
+//      divided by the ray count and written to the row's staging slot.
 // The rows are therefore emitted already in (row, column) order: no global
 // COO sort (src/cooSort.hpp:75-99) and no coo->csr pass are needed; a scan
 // of the row lengths and a gather place them into CSR.
@@ -28,6 +26,7 @@
 // explicit round-to-nearest intrinsics used on every exact path.
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstdint>
 
 #include "common.cuh"
@@ -99,11 +98,10 @@ struct RowTable {
   }
 };
 
-// Where the step walk adds a voxel's length.  KeyIndex tracks the voxel id
-// and adds to the row's hash table; DenseIndex tracks the voxel's slot in
-// the row's slab windows (below) and adds to it directly.  begin() takes the
-// ray's step directions, set() places the index at a voxel, advance() moves
-// it one voxel along the axis the walk steps (x if ax, else y if ay, else z).
+// Where the step walk adds a voxel's length: the voxel id, added to the row's
+// hash table.  begin() takes the ray's step directions, set() places the
+// index at a voxel, advance() moves it one voxel along the axis the walk
+// steps (x if ax, else y if ay, else z).
 template <int H>
 struct KeyIndex {
   const RowTable<H>* table;
@@ -119,58 +117,17 @@ struct KeyIndex {
   __device__ __forceinline__ void add(float L) const { table->add(key, L); }
 };
 
-// Slab windows of a row whose rays all cross the grid in the same direction
-// along the slab axis A (x or z): for every slab s of A the rays' voxels lie
-// in a window [ulo[s], ulo[s]+wu) x [vlo[s], vlo[s]+wv) of the other two
-// axes U < V (y, z for A = x; x, y for A = z), which holds wu*wv dense slots
-// from slot s*wu*wv on (slot = base[s] + iu*wv + iv).  A step in U moves the
-// slot by +-wv, in V by +-1, in A by dk[s] (the base difference to the next
-// slab in the rays' direction).  No key is stored or compared.
-template <int A>
-struct DenseIndex {
-  float* acc;
-  const int* base;
-  const int* dk;
-  int wv, nslots;
-  int slot, sa, ka, sta, ku, kv;
-  __device__ __forceinline__ void begin(const int step[3]) {
-    sta = step[A];
-    ku = step[A == 0 ? 1 : 0] * wv;
-    kv = step[A == 0 ? 2 : 1];
-  }
-  __device__ __forceinline__ void set(int i0, int i1, int i2) {
-    sa = A == 0 ? i0 : i2;
-    slot = A == 0 ? base[i0] + i1 * wv + i2 : base[i2] + i0 * wv + i1;
-    ka = dk[sa];
-  }
-  __device__ __forceinline__ void advance(bool ax, bool ay) {
-    if (A == 0) {
-      slot += ax ? ka : (ay ? ku : kv);
-      sa = ax ? sa + sta : sa;
-    } else {
-      slot += ax ? ku : (ay ? kv : ka);
-      sa = (ax || ay) ? sa : sa + sta;
-    }
-    ka = dk[sa];
-  }
-  __device__ __forceinline__ void add(float L) const {
-    // a slot outside the windows goes to the spare slot at nslots, which
-    // the row checks afterwards (no branch in the step loop)
-    atomicAdd(&acc[unsigned(slot) < unsigned(nslots) ? slot : nslots], L);
-  }
-};
-
 // Visits every grid voxel whose intersection length with ray r is positive.
 // A ray that crosses the planes of all three axes takes the step loop,
 // which adds the lengths through the index `ix`; any other ray takes the
 // general loop, which adds through emit(ix, iy, iz, L): a ray parallel to
 // the planes of some axis (start and end coordinate equal) leaves that axis
 // unconstrained, as the reference's masked min/max does, and every
-// candidate voxel along it gets the length.  UNROLL is the step loop's
-// unroll factor (the arithmetic of each step is the same for any).
-template <bool OISO, int UNROLL, class Emit, class Index>
+// candidate voxel along it gets the length.  Of those candidates the caller
+// gets every k_step-th from k_first on, so that a block can share them.
+template <bool OISO, class Emit, class Index>
 __device__ __forceinline__ void walk_ray(const DGeom& g, const Channel& ch, const float r[6], int part, Emit& emit,
-                                         Index& ix, int* bad_walk) {
+                                         Index& ix, int* bad_walk, int k_first, int k_step) {
   float dir[3];
   bool s[3];
 #pragma unroll
@@ -353,7 +310,7 @@ __device__ __forceinline__ void walk_ray(const DGeom& g, const Channel& ch, cons
     const float sq1 = float(step[1] > 0 ? s1 + 2 : 1 - s1);
     const float sq2 = float(step[2] > 0 ? s2 + 2 : 1 - s2);
     const float sprev = fmaxf(sl0, fmaxf(sl1, sl2));
-#pragma unroll UNROLL
+#pragma unroll 1
     for (int it = 0; it < guard_max; it++) {
       const float a_hi = fminf(hi0, fminf(hi1, hi2));
       // A voxel between two planes at the same parameter gets length 0; it
@@ -408,16 +365,16 @@ __device__ __forceinline__ void walk_ray(const DGeom& g, const Channel& ch, cons
       if (all3) {
         emit(id[0], id[1], id[2], L);
       } else {
-        int r0[3], r1[3];
+        int r0[3], m[3];
 #pragma unroll
         for (int d = 0; d < 3; d++) {
           r0[d] = s[d] ? id[d] : 0;
-          r1[d] = s[d] ? id[d] : g.n[d] - 1;
+          m[d] = s[d] ? 1 : g.n[d];
         }
-        for (int a = r0[0]; a <= r1[0]; a++)
-          for (int b = r0[1]; b <= r1[1]; b++)
-            for (int c = r0[2]; c <= r1[2]; c++)
-              if (candidate_test(g, ch, a, b, c)) emit(a, b, c, L);
+        for (int k = k_first; k < m[0] * m[1] * m[2]; k += k_step) {
+          const int a = r0[0] + k / (m[1] * m[2]), b = r0[1] + k / m[2] % m[1], c = r0[2] + k % m[2];
+          if (candidate_test(g, ch, a, b, c)) emit(a, b, c, L);
+        }
       }
     }
     if (!(a_hi < amax_g)) return;
@@ -463,85 +420,6 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* total, int* warp
   return before;
 }
 
-constexpr int kMaxSlabs = 256;
-
-// Dense slots of a row (floats) and the row kernel's dynamic shared memory:
-// the hash table's H keys and H sums, or the dense windows, whichever is
-// larger.  3H dense slots keep every row of the centred-cube workloads
-// dense; at H = 4096 the 48 KB still leave four CTAs per SM, which the
-// registers limit it to anyway.
-__host__ __device__ constexpr int dense_slots(int H) { return H <= 4096 ? 3 * H : 2 * H; }
-__host__ __device__ constexpr size_t row_smem_bytes(int H) {
-  return size_t(H) * 8 > size_t(dense_slots(H)) * 4 ? size_t(H) * 8 : size_t(dense_slots(H)) * 4;
-}
-
-// Row-level decision for the slab windows: both crystals' boxes (corner
-// AABBs) lie on opposite sides of the grid in x, so every ray of the row
-// crosses the whole grid in the same x direction (xdir) and lies in the
-// convex hull of the two boxes.
-__device__ inline void crystal_boxes(const Channel& ch, float lo[2][3], float hi[2][3]) {
-  for (int b = 0; b < 2; b++) {
-    const float* m = b == 0 ? ch.m0 : ch.m1;
-    for (int d = 0; d < 3; d++) {
-      lo[b][d] = INFINITY;
-      hi[b][d] = -INFINITY;
-    }
-    for (int c = 0; c < 8; c++) {
-      float p[3];
-      trafo_apply(m, float(c & 1), float((c >> 1) & 1), float((c >> 2) & 1), p);
-      for (int d = 0; d < 3; d++) {
-        lo[b][d] = fminf(lo[b][d], p[d]);
-        hi[b][d] = fmaxf(hi[b][d], p[d]);
-      }
-    }
-  }
-}
-
-// The voxel range along axis w that rays from box P (lower coordinate on
-// the slab axis a) to box Q can reach within the slab [c0, c1] of axis a: a
-// ray point at coordinate c is (1-t)*p + t*q with p in P, q in Q and t
-// between (c - bP)/(bQ - bP) and (c - aP)/(aQ - aP) ([aP, bP], [aQ, bQ] the
-// boxes' ranges along a), so its w lies between the extremes of the boxes'
-// w bounds at those t, at both slab faces.  One voxel of margin on each
-// side covers rounding.
-__device__ inline void slab_window(const DGeom& g, int a, const float plo[3], const float phi[3],
-                                   const float qlo[3], const float qhi[3], float c0, float c1, int w, int* ilo,
-                                   int* ihi) {
-  float wlo = INFINITY, whi = -INFINITY;
-#pragma unroll
-  for (int e = 0; e < 2; e++) {
-    const float c = e == 0 ? c0 : c1;
-    const float t1 = (c - phi[a]) / (qhi[a] - phi[a]);
-    const float t2 = (c - plo[a]) / (qlo[a] - plo[a]);
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const float t = k == 0 ? t1 : t2;
-      wlo = fminf(wlo, plo[w] + t * (qlo[w] - plo[w]));
-      whi = fmaxf(whi, phi[w] + t * (qhi[w] - phi[w]));
-    }
-  }
-  const int n = axis_n(g, w);
-  int lo = int(floorf((wlo - axis_o(g, w)) / axis_d(g, w))) - 1;
-  int hi = int(floorf((whi - axis_o(g, w)) / axis_d(g, w))) + 1;
-  lo = min(max(lo, 0), n - 1);
-  hi = min(max(hi, 0), n - 1);
-  *ilo = lo;
-  *ihi = max(lo, hi);
-}
-
-// The dense kernel's step-loop unroll factor by row capacity, measured on
-// full builds: 6 at H = 4096 (70^3 x 5.14M channels: 2.04 s unrolled 1,
-// 2.00 s by 2, 1.86 s by 4, 1.81 s by 6 and by 8; 8 spills), none at
-// H = 8192 (100^3 x 1.71M channels: 1.23 s unrolled 1, 1.25 s by 4, 1.32 s
-// by 6, 1.37 s by 8) nor at H = 2048 (40^3 x 143K channels: 8-9 ms either
-// way, and unrolled it spills).
-constexpr int dense_walk_unroll(int H) { return H == 4096 ? 6 : 1; }
-
-// Row status the dense kernel leaves for the table kernel: the row is to be
-// built with the hash table (it does not qualify for dense windows, or a
-// ray left its windows).
-constexpr int kRowToTable = -2;
-
 // Bitonic sort of (keys, vals)[0, total) by key in shared memory (npad =
 // the next power of two, padded with INT_MAX), then written to the row's
 // staging slot and its length to *row_nnz.  Every thread of the CTA calls it.
@@ -578,40 +456,365 @@ __device__ void sort_and_write(int* keys, float* vals, int total, int32_t* __res
   if (tid == 0) *row_nnz = total;
 }
 
-// Dense kernel: one CTA per row whose two crystals lie on opposite sides of
-// the grid along x or z (generated rays only).  Every ray of such a row
-// crosses the grid in the same direction along that slab axis and lies in
-// the convex hull of the two crystal boxes, so the voxels its rays reach lie
-// in per-slab windows, and the lengths are summed into dense slots of those
-// windows: no key is stored, loaded or compared.  The voxels with a positive
-// sum that pass the cylinder test are written in column order (x slabs are
-// in column order already; z slabs are sorted).  A row that does not
-// qualify, whose windows exceed dense_slots(H), or one of whose rays leaves
-// its windows gets row_nnz = kRowToTable and is built by sm_table_kernel.
-// Why the windows hold every voxel a ray visits: the hull bound is exact in
-// real arithmetic, the walk visits voxels adjacent to the real ray's voxels
-// at worst (rounding at plane ties), and the windows have a margin of one
-// voxel on each side; the spare slot and the compaction's decode check
-// catch a slot outside the windows' range regardless.
-template <int H, int T, bool OISO>
-__global__ void __launch_bounds__(T) sm_dense_kernel(DGeom g, const float2* __restrict__ sincos,
-                                                     const int32_t* __restrict__ cnl_ids, int64_t row0, int nrays,
-                                                     uint32_t seed, int32_t* __restrict__ st_col,
-                                                     float* __restrict__ st_val, int32_t* __restrict__ row_nnz,
-                                                     int32_t* __restrict__ flags, int32_t* __restrict__ reasons) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  float* acc = reinterpret_cast<float*>(smem);  // dense_slots(H) slots + the spare one
-  int* keys = reinterpret_cast<int*>(smem);     // z slabs: the row's entries for the sort
-  float* vals = reinterpret_cast<float*>(smem + H * sizeof(int));
-  __shared__ Channel ch;
-  __shared__ int bad_walk, dense_fail, win_u, win_v, sax, sdir;
-  __shared__ float box_lo[2][3], box_hi[2][3];
-  __shared__ int warp_sums[32];
-  __shared__ int ulo[kMaxSlabs], vlo[kMaxSlabs], sbase[kMaxSlabs], sdk[kMaxSlabs];
+// ---------------------------------------------------------------------------
+// Slab kernel: one thread owns one slab of the grid
+// ---------------------------------------------------------------------------
+//
+// When both crystals of a row lie on opposite sides of the grid along x or z
+// (the slab axis A), every ray of the row crosses the grid in the same
+// direction along A.  A thread then owns kSlabs neighbouring slabs of A (the
+// voxels between two planes of A) for one of G groups of the row's rays, and
+// for each of its rays finds the segments inside its slabs on its own: the
+// parameters of the slabs' planes, and in each slab of the one plane of each
+// other axis (u < v) that the ray can cross there.  What bounds it is
+// instruction issue (no HBM traffic but the finished row, no contraction):
+//
+//  * no order between the slabs of a ray is needed, so there is no walk state,
+//    no choice of the next axis by selects, no divergence between long and
+//    short rays (31 of 32 lanes active; 25 in a walk);
+//  * u and v, and two planes of A, go through the same operations as packed
+//    pairs (add/mul/fma.rn.f32x2, each result correctly rounded; 7 % faster
+//    than the scalar operations);
+//  * a thread's sums are its own (one shared-memory column per thread), so
+//    they are plain loads and stores without bank conflicts: a shared-memory
+//    float atomic is a compare-and-swap loop;
+//  * three slabs share the ray's loads and their inner planes.
+//
+// A ray costs the same in any direction, while a walk takes one step per
+// crossing (75 at 0 degrees, ~110 at 45 for 70^3 voxels).  Measured against
+// the walk into dense windows with shared-memory atomics that it replaces:
+// 60,000 rows of 70^3 x 1000 rays 19.4 -> 13.5 ms, 12,345 rows of 100^3 x 999
+// rays 12.6 -> 5.1 ms (half of those rows did not fit the dense windows).
+// Main loop, ~54 issue slots per (ray, slab) and as many again for half of
+// the packed operations: 2/3 of the time; ray generation, set-up and
+// compaction the rest.
+//
+// Exactness.  The plane parameters are computed with the operations of
+// walk_ray (and of the reference), so each is the same float.  A segment of
+// a voxel lies between consecutive plane parameters in their float order,
+// which are monotone in the plane index; a segment exists where they
+// increase strictly.  Within a slab [lo, hi] a thread takes the first plane
+// of u and of v that can come after lo: the index is computed from an
+// approximate coordinate lowered by eps, a bound on its rounding error, so
+// that every earlier plane's float parameter is at most lo.  That plane may
+// lie before lo too (its segment is then empty), and a second plane of an
+// axis may lie before hi: whenever that is possible (within 2 eps) the
+// thread walks its slab plane by plane instead (slab_walk, 3 % of the time:
+// planes within eps, and rays steeper than one voxel per slab).
 
-  const int tid = threadIdx.x;
-  const int64_t li = row0 + blockIdx.x;
-  const int cnl = cnl_ids[li];
+using f32x2 = unsigned long long;
+
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// Two quotients a / b, each as div_rcp: nb = -b, y = RN(1 / b).
+__device__ __forceinline__ f32x2 div_rcp2(f32x2 a, f32x2 nb, f32x2 y) {
+  f32x2 q = mul2(a, y);
+  f32x2 r = fma2(q, nb, a);
+  q = fma2(r, y, q);
+  r = fma2(q, nb, a);
+  return fma2(r, y, q);
+}
+
+// A ray as the slab threads read it (16-byte broadcast loads), signed by the
+// ray's step directions so that plane indices grow along it (q = step * i,
+// and the pitch carries the sign back: q * p == i * d exactly).
+struct alignas(16) SlabRay {
+  float nr0a[2];        // -start along A, twice
+  float rca[2];         // RN(1/direction) along A, twice
+  float nda[2];         // -direction along A, twice
+  float amin, amax;     // the ray's parameter range inside the grid
+  float g[2];           // voxels per unit parameter along u, v
+  float f[2];           // signed coordinate at parameter 0, - eps + 1/2
+  float p[2];           // signed pitch along u, v
+  float nr0[2];         // -start along u, v
+  float rc[2];          // RN(1/direction) along u, v
+  float nd[2];          // -direction along u, v
+  float w[2];           // parameter from one plane to the next, less 2 eps of it
+  float len;            // |end - start|
+  unsigned c;           // the ray's part of the byte offset (below)
+  unsigned k[2];        // byte step of a voxel step along u, v
+  float nzero[2];       // -0, twice: the plane's q * p is taken as fma(q, p, -0)
+                        // (the assembler contracts mul.rn.f32x2 with the add.rn.f32x2
+                        // after it into one rounding, unlike the scalar pair)
+};
+static_assert(sizeof(SlabRay) == 112, "seven 16-byte loads");
+
+constexpr int kSlabs = 3;               // neighbouring slabs a thread owns (odd: an even number of planes)
+constexpr int kSlabBatch = 192;              // rays staged in shared memory at a time
+constexpr float kIndexMagic = 12582912.f;  // 1.5 * 2^23: adding it rounds to an integer held in the low mantissa bits
+constexpr unsigned kIndexBits = 0x4B400000u;
+
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// Adds the length `d * len` to the float `off` bytes into `acc`: one rounding
+// (a positive length stays positive).
+__device__ __forceinline__ void slab_add(unsigned char* acc, unsigned off, float d, float len) {
+  float* p = reinterpret_cast<float*>(acc + off);
+  *p = __fmaf_rn(d, len, *p);
+}
+
+// The slow path: ray R's segments in one slab between the parameters a0 and
+// a1 of its planes, plane by plane.
+__device__ __noinline__ void slab_walk(const SlabRay* __restrict__ R, float a0, float a1, unsigned off, float ou,
+                                       float ov, unsigned spare, unsigned char* acc, int* bad_walk) {
+  float cur = fmaxf(a0, R->amin);
+  const float hi = fminf(a1, R->amax), len = R->len;
+  const float mu = RFADD(__fmaf_rn(R->g[0], cur, R->f[0]), kIndexMagic);
+  const float mv = RFADD(__fmaf_rn(R->g[1], cur, R->f[1]), kIndexMagic);
+  float cu = RFSUB(mu, kIndexMagic), cv = RFSUB(mv, kIndexMagic);
+  auto plane = [&](int k, float c, float o) {
+    return div_rcp(RFADD(RFADD(RFMUL(c, R->p[k]), o), R->nr0[k]), -R->nd[k], R->rc[k]);
+  };
+  float hu = plane(0, cu, ou), hv = plane(1, cv, ov);
+  off += unsigned(__float_as_int(mu)) * R->k[0] + unsigned(__float_as_int(mv)) * R->k[1] + R->c;
+#pragma unroll 1
+  for (int guard = 0; guard < 4096; guard++) {
+    const float e = min3(hu, hv, hi);
+    if (e > cur) {
+      slab_add(acc, min(off, spare), RFSUB(e, cur), len);
+      cur = e;
+    }
+    if (!(e < hi)) return;
+    if (hu <= hv) {
+      cu = RFADD(cu, 1.0f);
+      off += R->k[0];
+      hu = plane(0, cu, ou);
+    } else {
+      cv = RFADD(cv, 1.0f);
+      off += R->k[1];
+      hv = plane(1, cv, ov);
+    }
+  }
+  *bad_walk = 1;
+}
+
+// The segments of ray R inside the thread's kSlabs slabs: pl = the planes
+// before and after them in the ray's order, off0 = per slab the thread's part
+// of the byte offset, o2 = the origin along (u, v), spare = the byte offset of
+// the thread's spare slots, which take what an offset beyond the windows would
+// hold (one per segment, `step` bytes apart, so that the three loads of a slab
+// can go ahead of its stores).
+__device__ __forceinline__ void slab_step(const SlabRay* __restrict__ R, const f32x2 (&pl)[(kSlabs + 2) / 2],
+                                          const unsigned (&off0)[kSlabs], f32x2 o2, unsigned spare, unsigned step,
+                                          unsigned char* acc, int* bad_walk) {
+  const ulonglong2* q = reinterpret_cast<const ulonglong2*>(R);
+  const ulonglong2 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4], q5 = q[5], q6 = q[6];
+  float a[kSlabs + 2], amin, amax, len, cf;
+#pragma unroll
+  for (int j = 0; j < (kSlabs + 2) / 2; j++) unpack2(div_rcp2(add2(pl[j], q0.x), q1.x, q0.y), a[2 * j], a[2 * j + 1]);
+  unpack2(q1.y, amin, amax);
+  unpack2(q5.y, len, cf);
+  const unsigned c = unsigned(__float_as_int(cf));
+  const uint2 k = make_uint2(unsigned(q6.x), unsigned(q6.x >> 32));
+  const f32x2 magic = pack2(kIndexMagic, kIndexMagic), nmagic = pack2(-kIndexMagic, -kIndexMagic);
+  bool slow[kSlabs];
+  float d1[kSlabs], d2[kSlabs], d3[kSlabs];
+  unsigned o1[kSlabs], o2_[kSlabs], o3[kSlabs];
+#pragma unroll
+  for (int j = 0; j < kSlabs; j++) {
+    // hi == lo where the ray is not inside the grid: three empty segments
+    const float lo = fmaxf(a[j], amin);
+    float hi = fmaxf(fminf(a[j + 1], amax), lo);
+    const f32x2 m = add2(fma2(q2.x, pack2(lo, lo), q2.y), magic);
+    const f32x2 qi = add2(m, nmagic);
+    const f32x2 h = div_rcp2(add2(add2(fma2(qi, q3.x, q6.y), o2), q3.y), q4.y, q4.x);
+    float hu, hv, wu, wv, mu, mv;
+    unpack2(h, hu, hv);
+    unpack2(add2(h, q5.x), wu, wv);
+    unpack2(m, mu, mv);
+    const unsigned off = unsigned(__float_as_int(mu)) * k.x + (unsigned(__float_as_int(mv)) * k.y + (c + off0[j]));
+    slow[j] = fminf(wu, wv) < hi;
+    hi = slow[j] ? lo : hi;
+    const float e1 = fmaxf(min3(hu, hv, hi), lo), e2 = fminf(max3(hu, hv, lo), hi);
+    d1[j] = RFSUB(e1, lo);
+    d2[j] = RFSUB(e2, e1);
+    d3[j] = RFSUB(hi, e2);
+    o1[j] = min(off, spare);
+    o2_[j] = min(off + (hu <= hv ? k.x : k.y), spare + step);
+    o3[j] = min(off + k.x + k.y, spare + 2 * step);
+  }
+#pragma unroll
+  for (int j = 0; j < kSlabs; j++) {
+    float* p1 = reinterpret_cast<float*>(acc + o1[j]);
+    float* p2 = reinterpret_cast<float*>(acc + o2_[j]);
+    float* p3 = reinterpret_cast<float*>(acc + o3[j]);
+    const float v1 = *p1, v2 = *p2, v3 = *p3;
+    *p1 = __fmaf_rn(d1[j], len, v1);
+    *p2 = __fmaf_rn(d2[j], len, v2);
+    *p3 = __fmaf_rn(d3[j], len, v3);
+  }
+  bool any = slow[0];
+#pragma unroll
+  for (int j = 1; j < kSlabs; j++) any = any || slow[j];
+  if (any) {
+    float ou, ov;
+    unpack2(o2, ou, ov);
+#pragma unroll
+    for (int j = 0; j < kSlabs; j++)
+      if (slow[j]) slab_walk(R, a[j], a[j + 1], off0[j], ou, ov, spare, acc, bad_walk);
+  }
+}
+
+// Fills R for the ray r of the row (slab axis A, direction sdir along it);
+// false where the row is to go to the table kernel: a direction component
+// that is zero or out of the reciprocal's range, or coordinates so large
+// against a voxel that eps would not be small.
+__device__ __forceinline__ bool slab_ray(const DGeom& g, const float r[6], int A, int sdir, int wv, unsigned stride,
+                                         SlabRay* R) {
+  float dir[3], rc[3];
+  float amin = -INFINITY, amax = INFINITY;
+  bool ok = true;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    dir[d] = RFSUB(r[3 + d], r[d]);
+    ok = ok && fabsf(dir[d]) >= 1e-30f && fabsf(dir[d]) <= 1e30f;
+  }
+  float4 q[7];
+  if (ok) {
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      rc[d] = __frcp_rn(dir[d]);
+      const float a0 = div_rcp(RFSUB(RFADD(g.o[d], RFMUL(0.f, g.d[d])), r[d]), dir[d], rc[d]);
+      const float a1 = div_rcp(RFSUB(RFADD(g.o[d], RFMUL(float(g.n[d]), g.d[d])), r[d]), dir[d], rc[d]);
+      amin = fmaxf(amin, fminf(a0, a1));
+      amax = fminf(amax, fmaxf(a0, a1));
+    }
+    const float da = A == 0 ? dir[0] : dir[2], ra = A == 0 ? r[0] : r[2], rca = A == 0 ? rc[0] : rc[2];
+    ok = sdir > 0 ? da > 0.f : da < 0.f;
+    q[0] = make_float4(-ra, -ra, rca, rca);
+    q[1] = make_float4(-da, -da, amin, amax);
+    float G[2], F[2], P[2], X[2], RC[2], ND[2], Wd[2];
+    unsigned c = 0, K[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      // u = y, v = z for A = x; u = x, v = y for A = z
+      const float o = k == 0 ? (A == 0 ? g.o[1] : g.o[0]) : (A == 0 ? g.o[2] : g.o[1]);
+      const float d = k == 0 ? (A == 0 ? g.d[1] : g.d[0]) : (A == 0 ? g.d[2] : g.d[1]);
+      const int n = k == 0 ? (A == 0 ? g.n[1] : g.n[0]) : (A == 0 ? g.n[2] : g.n[1]);
+      const float x = k == 0 ? (A == 0 ? r[1] : r[0]) : (A == 0 ? r[2] : r[1]);
+      const float dk = k == 0 ? (A == 0 ? dir[1] : dir[0]) : (A == 0 ? dir[2] : dir[1]);
+      const float rk = k == 0 ? (A == 0 ? rc[1] : rc[0]) : (A == 0 ? rc[2] : rc[1]);
+      const bool up = dk > 0.f;
+      const float inv = __fdividef(1.0f, d);
+      const float f = (up ? x - o : o - x) * inv;
+      G[k] = fabsf(dk) * inv;
+      // the roundings of f + a*G and of the plane parameters, in voxels: at
+      // most seven of 2^-24 of each of these magnitudes
+      const float eps = 4.2e-7f * (2.f * fabsf(f) + G[k] + 2.f * fabsf(o) * inv + float(n) + 2.f);
+      ok = ok && eps <= 0.01f;
+      F[k] = (0.5f - eps) + f;
+      P[k] = up ? d : -d;
+      X[k] = -x;
+      RC[k] = rk;
+      ND[k] = -dk;
+      Wd[k] = (1.0f - 2.f * eps) * (fabsf(rk) * d);
+      const unsigned step = k == 0 ? stride * unsigned(wv) : stride;
+      K[k] = up ? step : 0u - step;
+      // the voxel before plane q is q - 1 going up, -q going down; the
+      // indices come with kIndexBits on them
+      c -= kIndexBits * K[k] + (up ? step : 0u);
+    }
+    q[2] = make_float4(G[0], G[1], F[0], F[1]);
+    q[3] = make_float4(P[0], P[1], X[0], X[1]);
+    q[4] = make_float4(RC[0], RC[1], ND[0], ND[1]);
+    q[5] = make_float4(Wd[0], Wd[1], norm3_exact(dir[0], dir[1], dir[2]), __uint_as_float(c));
+    q[6] = make_float4(__uint_as_float(K[0]), __uint_as_float(K[1]), -0.f, -0.f);
+  }
+  if (!ok) {
+#pragma unroll
+    for (int k = 0; k < 7; k++) q[k] = make_float4(0.f, 0.f, 0.f, 0.f);  // every parameter 0: empty segments only
+  }
+  float4* out = reinterpret_cast<float4*>(R);
+#pragma unroll
+  for (int k = 0; k < 7; k++) out[k] = q[k];
+  return ok;
+}
+
+// i / d for i, d < 2^16 from m = div_magic(d): exact, since the magic number
+// is off by less than d in 2^32 and i * d < 2^32.
+__device__ __forceinline__ unsigned div_magic(int d) { return 0xffffffffu / unsigned(d) + 1u; }
+__device__ __forceinline__ int div_by(int i, int d, unsigned m) { return d == 1 ? i : int(__umulhi(unsigned(i), m)); }
+
+// Row status the slab kernel leaves for the table kernel: the row is to be
+// built with the hash table.
+constexpr int kRowToTable = -2;
+
+constexpr int kMaxSlabs = 256;
+
+constexpr int kSlabThreads = 192, kSlabBlocks = 3;  // most threads, blocks per SM
+
+// Launch shape of the slab kernel on a grid: threads per block, floats of
+// the sums and of the ray staging in dynamic shared memory.
+struct SlabShape {
+  int threads = 0;
+  int acc_floats = 0;
+  int stage_floats = 0;
+  size_t smem() const { return size_t(acc_floats + stage_floats) * 4; }
+};
+
+// One block per row.  The sums of the row's windows (per slab of A the
+// voxels [ulo, ulo+wu) x [vlo, vlo+wv) that the crystals' hull can reach)
+// are kept per thread: slot w of thread t at acc[w * S + t], S = the threads
+// in use rounded up to a warp.  A row with more slots per slab than fit runs
+// with fewer groups of rays; one whose slots do not fit one group, that has
+// no slab axis, or one of whose rays needs the general walk gets row_nnz =
+// kRowToTable and is built by sm_table_kernel.
+//
+// The windows hold every voxel a ray visits: a ray lies in the convex hull
+// of the two crystals, the windows are the hull's extents at the slab's two
+// faces taken over all pairs of corners, with 0.02 voxel of margin against
+// rounding (the rays' eps is at most 0.01 voxel).  An offset outside the
+// row's slots goes to the thread's spare slot and a positive sum that
+// decodes outside the grid is noticed: both send the row to the table.
+__global__ void __launch_bounds__(kSlabThreads, kSlabBlocks)
+    sm_slab_kernel(DGeom g, const float2* __restrict__ sincos, const int32_t* __restrict__ cnl_ids, int64_t row0,
+                   int nrays, uint32_t seed, int H, int acc_floats, int stage_floats, int32_t* __restrict__ st_col,
+                   float* __restrict__ st_val, int32_t* __restrict__ row_nnz, int32_t* __restrict__ flags,
+                   int32_t* __restrict__ reasons) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  float* acc = reinterpret_cast<float*>(smem);
+  float* stage = acc + acc_floats;  // the rays of a batch, then the row's sums
+  SlabRay* rays = reinterpret_cast<SlabRay*>(stage);
+  __shared__ Channel ch;
+  __shared__ int bad_walk, to_table, outside, win_u, win_v;
+  __shared__ float corner_x[2][4], corner_z[2][4], corner_y[2][2];
+  __shared__ int warp_sums[32];
+  __shared__ short ulo[kMaxSlabs], vlo[kMaxSlabs];
+  __shared__ int zbox[4];
+
+  const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5, NW = T >> 5;
+  const int cnl = cnl_ids[row0 + blockIdx.x];
   if (cnl < 0 || cnl >= num_channels(g)) {
     if (tid == 0) {
       row_nnz[blockIdx.x] = -1;
@@ -619,107 +822,167 @@ __global__ void __launch_bounds__(T) sm_dense_kernel(DGeom g, const float2* __re
     }
     return;
   }
-  const int nyz = g.n[1] * g.n[2];
-  const int nz = g.n[2];
+  auto table = [&](int why) {  // called by every thread, or by one
+    if (tid == 0) {
+      row_nnz[blockIdx.x] = kRowToTable;
+      if (reasons) atomicAdd(reasons + why, 1);
+    }
+  };
   if (tid == 0) {
     channel_setup(g, sincos, cnl, ch);
     bad_walk = 0;
-    dense_fail = 0;
+    to_table = 0;
+    outside = 0;
     win_u = 0;
     win_v = 0;
-    crystal_boxes(ch, box_lo, box_hi);
-    // the slab axis: of x and z, the one along which the crystals lie on
-    // opposite sides of the grid, the channel's dominant direction first
-    // (its windows are the narrowest)
-    int axis = -1, dir = 0;
-    const int first = fabsf(ch.ab[0]) >= fabsf(ch.ab[2]) ? 0 : 2;
-    for (int k = 0; k < 2 && axis < 0; k++) {
-      const int a = k == 0 ? first : 2 - first;
-      if (axis_n(g, a) > kMaxSlabs) continue;
-      const float c0 = axis_o(g, a), c1 = axis_o(g, a) + float(axis_n(g, a)) * axis_d(g, a);
-      const float m = 1e-6f * (1.0f + fabsf(c0) + fabsf(c1));
-      if (box_hi[0][a] + m < c0 && box_lo[1][a] - m > c1) dir = 1;
-      if (box_hi[1][a] + m < c0 && box_lo[0][a] - m > c1) dir = -1;
-      if (dir != 0) axis = a;
-    }
-    sax = axis;
-    sdir = dir;
+    zbox[0] = zbox[2] = INT_MAX;
+    zbox[1] = zbox[3] = INT_MIN;
+  } else if (tid >= 32) {
+    // the other warps clear the sums meanwhile
+    float4* a4 = reinterpret_cast<float4*>(acc);
+    for (int i = tid - 32; i < acc_floats / 4; i += T - 32) a4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __syncthreads();
-  const int A = sax;
-  if (A < 0) {
-    if (tid == 0) {
-      row_nnz[blockIdx.x] = kRowToTable;
-      if (reasons) atomicAdd(reasons + 0, 1);
+  if (tid < 8) {
+    // the crystals are boxes rotated about y: four corners in (x, z), two
+    // bounds in y
+    const int b = tid >> 2, c = tid & 3;
+    float p[3];
+    trafo_apply(b == 0 ? ch.m0 : ch.m1, float(c & 1), float(c >> 1), float(c >> 1), p);
+    corner_x[b][c] = p[0];
+    corner_z[b][c] = p[2];
+    if ((c & 1) == 0) corner_y[b][c >> 1] = p[1];
+  }
+  __syncthreads();
+  // the slab axis: of x and z, the one along which the crystals lie on
+  // opposite sides of the grid, the channel's dominant direction first
+  int A = -1, sdir = 0;
+  {
+    const int first = fabsf(ch.ab[0]) >= fabsf(ch.ab[2]) ? 0 : 2;
+    for (int k = 0; k < 2 && A < 0; k++) {
+      const int a = k == 0 ? first : 2 - first;
+      if (axis_n(g, a) > kMaxSlabs) continue;
+      const float* p = a == 0 ? corner_x[0] : corner_z[0];
+      const float* q = a == 0 ? corner_x[1] : corner_z[1];
+      const float plo = fminf(fminf(p[0], p[1]), fminf(p[2], p[3])), phi = fmaxf(fmaxf(p[0], p[1]), fmaxf(p[2], p[3]));
+      const float qlo = fminf(fminf(q[0], q[1]), fminf(q[2], q[3])), qhi = fmaxf(fmaxf(q[0], q[1]), fmaxf(q[2], q[3]));
+      const float c0 = axis_o(g, a), c1 = axis_o(g, a) + float(axis_n(g, a)) * axis_d(g, a);
+      const float m = 1e-6f * (1.0f + fabsf(c0) + fabsf(c1));
+      if (phi + m < c0 && qlo - m > c1) sdir = 1;
+      if (qhi + m < c0 && plo - m > c1) sdir = -1;
+      if (sdir != 0) A = a;
     }
+  }
+  if (A < 0) {
+    table(0);
+    return;
+  }
+  const int na = axis_n(g, A);
+  if (na > T * kSlabs) {
+    table(1);
     return;
   }
   const int iu_ax = A == 0 ? 1 : 0, iv_ax = A == 0 ? 2 : 1;
-  const int na = axis_n(g, A);
   {
-    const int p = sdir > 0 ? 0 : 1;  // the box at the lower coordinate along A
+    int wu_max = 0, wv_max = 0;
     for (int sl = tid; sl < na; sl += T) {
+      const float* pa = A == 0 ? corner_x[0] : corner_z[0];
+      const float* qa = A == 0 ? corner_x[1] : corner_z[1];
+      const float* pw = A == 0 ? corner_z[0] : corner_x[0];
+      const float* qw = A == 0 ? corner_z[1] : corner_x[1];
       const float c0 = axis_o(g, A) + float(sl) * axis_d(g, A), c1 = axis_o(g, A) + float(sl + 1) * axis_d(g, A);
-      int u0, u1, v0, v1;
-      slab_window(g, A, box_lo[p], box_hi[p], box_lo[1 - p], box_hi[1 - p], c0, c1, iu_ax, &u0, &u1);
-      slab_window(g, A, box_lo[p], box_hi[p], box_lo[1 - p], box_hi[1 - p], c0, c1, iv_ax, &v0, &v1);
-      ulo[sl] = u0;
-      vlo[sl] = v0;
-      atomicMax(&win_u, u1 - u0 + 1);
-      atomicMax(&win_v, v1 - v0 + 1);
+      float wlo = INFINITY, whi = -INFINITY, tlo = INFINITY, thi = -INFINITY;
+#pragma unroll 4
+      for (int ij = 0; ij < 16; ij++) {
+        const int i = ij >> 2, j = ij & 3;
+        const float inv = __fdividef(1.0f, qa[j] - pa[i]);
+        const float t0 = (c0 - pa[i]) * inv, t1 = (c1 - pa[i]) * inv;
+        const float w0 = pw[i] + t0 * (qw[j] - pw[i]), w1 = pw[i] + t1 * (qw[j] - pw[i]);
+        wlo = fminf(wlo, fminf(w0, w1));
+        whi = fmaxf(whi, fmaxf(w0, w1));
+        tlo = fminf(tlo, fminf(t0, t1));
+        thi = fmaxf(thi, fmaxf(t0, t1));
+      }
+      const float dy0 = corner_y[1][0] - corner_y[0][0], dy1 = corner_y[1][1] - corner_y[0][1];
+      const float ylo = corner_y[0][0] + fminf(tlo * dy0, thi * dy0);
+      const float yhi = corner_y[0][1] + fmaxf(tlo * dy1, thi * dy1);
+      auto range = [&](int ax, float lo, float hi, int* first) {
+        const int n = axis_n(g, ax);
+        const float inv = __fdividef(1.0f, axis_d(g, ax));
+        const int a = int(floorf((lo - axis_o(g, ax)) * inv - 0.02f)), b = int(floorf((hi - axis_o(g, ax)) * inv + 0.02f));
+        const int l = min(max(a, 0), n - 1);
+        *first = l;
+        return max(min(max(b, 0), n - 1) - l, 0) + 1;
+      };
+      int y0, w0;
+      const int ny = range(1, ylo, yhi, &y0);
+      const int nw = range(A == 0 ? 2 : 0, wlo, whi, &w0);
+      wu_max = max(wu_max, A == 0 ? ny : nw);
+      wv_max = max(wv_max, A == 0 ? nw : ny);
+      ulo[sl] = short(A == 0 ? y0 : w0);
+      vlo[sl] = short(A == 0 ? w0 : y0);
+    }
+    wu_max = __reduce_max_sync(0xffffffffu, wu_max);
+    wv_max = __reduce_max_sync(0xffffffffu, wv_max);
+    if (lane == 0 && wu_max > 0) {
+      atomicMax(&win_u, wu_max);
+      atomicMax(&win_v, wv_max);
     }
   }
   __syncthreads();
-  const int wu = win_u, wv = win_v;
-  const int wuv = wu * wv;
-  if (!((long long)na * wuv < (long long)dense_slots(H))) {  // + the spare slot
-    if (tid == 0) {
-      row_nnz[blockIdx.x] = kRowToTable;
-      if (reasons) atomicAdd(reasons + 1, 1);
-    }
+  // a voxel's offset and those one step on along u, v and both are four
+  // different ones (slab_step loads three before it stores): wv is not 1
+  const int wu = win_u, wv = max(win_v, 2), W = wu * wv;
+  const int nt = (na + kSlabs - 1) / kSlabs;  // threads of a group
+  int G = T / nt;
+  G = min(G, kSlabBatch);
+  while (G > 0 && (long long)(kSlabs * W + 3) * ((G * nt + 31) & ~31) > (long long)acc_floats) G--;
+  const int Wp = W | 1;  // odd: slots of neighbouring slabs fall into different banks
+  if (G == 0 || (long long)na * Wp > (long long)stage_floats) {
+    table(1);
     return;
   }
-  const int nslots = na * wuv;
-  for (int sl = tid; sl < na; sl += T) {
-    const int b = sl * wuv - ulo[sl] * wv - vlo[sl];
-    const int nb = sdir > 0 ? sl + 1 : sl - 1;
-    const int bn = (nb >= 0 && nb < na) ? nb * wuv - ulo[nb] * wv - vlo[nb] : b;
-    sbase[sl] = b;
-    sdk[sl] = bn - b;
-  }
-  for (int i = tid; i <= nslots; i += T) acc[i] = 0.f;
-  __syncthreads();
+  const int S = (G * nt + 31) & ~31;
+  const int grp = tid / nt, s0 = (tid - grp * nt) * kSlabs;
 
+  // the thread's slabs, in the rays' order; those past the last have two
+  // equal planes
+  const bool works = grp < G;
+  f32x2 pl[(kSlabs + 2) / 2];
+  unsigned off0[kSlabs];
   {
-    auto emit = [&](int ix, int iy, int iz, float L) {
-      const int sa = A == 0 ? ix : iz;
-      const int u = (A == 0 ? iy : ix) - ulo[sa], v = (A == 0 ? iz : iy) - vlo[sa];
-      if (unsigned(u) < unsigned(wu) && unsigned(v) < unsigned(wv))
-        atomicAdd(&acc[sa * wuv + u * wv + v], L);
-      else
-        dense_fail = 1;
-    };
-    // start offsets: the thread index bit-reversed, so that neighbouring
-    // lanes start far apart along the ray
-    const int part = int(__brev(threadIdx.x) >> 24);
-    if (A == 0) {
-      DenseIndex<0> dix{acc, sbase, sdk, wv, nslots};
-      for (int ray = tid; ray < nrays; ray += T) {
-        float r[6];
-        make_ray(ch, seed, cnl, ray, r);
-        if (sdir > 0 ? !(RFSUB(r[3], r[0]) > 0.f) : !(RFSUB(r[3], r[0]) < 0.f)) dense_fail = 1;
-        walk_ray<OISO, dense_walk_unroll(H)>(g, ch, r, part, emit, dix, &bad_walk);
-      }
-    } else {
-      DenseIndex<2> dix{acc, sbase, sdk, wv, nslots};
-      for (int ray = tid; ray < nrays; ray += T) {
-        float r[6];
-        make_ray(ch, seed, cnl, ray, r);
-        if (sdir > 0 ? !(RFSUB(r[5], r[2]) > 0.f) : !(RFSUB(r[5], r[2]) < 0.f)) dense_fail = 1;
-        walk_ray<OISO, dense_walk_unroll(H)>(g, ch, r, part, emit, dix, &bad_walk);
-      }
+    float p[kSlabs + 2];
+    p[kSlabs + 1] = 0.f;
+#pragma unroll
+    for (int j = 0; j <= kSlabs; j++)
+      p[j] = RFADD(axis_o(g, A), RFMUL(float(min(sdir > 0 ? s0 + j : s0 + kSlabs - j, na)), axis_d(g, A)));
+#pragma unroll
+    for (int j = 0; j < (kSlabs + 2) / 2; j++) pl[j] = pack2(p[2 * j], p[2 * j + 1]);
+#pragma unroll
+    for (int j = 0; j < kSlabs; j++) {
+      const int k = sdir > 0 ? j : kSlabs - 1 - j, sl = min(s0 + k, na - 1);
+      off0[j] = unsigned((k * W * S + tid) * 4) - unsigned(ulo[sl] * wv + vlo[sl]) * unsigned(S * 4);
     }
   }
+  const unsigned spare = unsigned((kSlabs * W * S + (works ? tid : 0)) * 4);
+  const f32x2 o2 = pack2(axis_o(g, iu_ax), axis_o(g, iv_ax));
+  const int per = kSlabBatch / G * G;  // as many rays for every group
+  for (int base = 0; base < nrays; base += per) {
+    const int cnt = min(per, nrays - base);
+    __syncthreads();  // the batch before is done with
+    for (int i = tid; i < cnt; i += T) {
+      float r[6];
+      make_ray(ch, seed, cnl, base + i, r);
+      if (!slab_ray(g, r, A, sdir, wv, unsigned(S * 4), rays + i)) to_table = 1;
+    }
+    __syncthreads();
+    if (works)
+      for (int i = grp; i < cnt; i += G)
+        slab_step(rays + i, pl, off0, o2, spare, unsigned(S * 4), smem, &bad_walk);
+  }
+  if (works)
+    for (int k = 0; k < 3; k++)
+      if (acc[(kSlabs * W + k) * S + tid] != 0.f) to_table = 1;
   __syncthreads();
   if (bad_walk) {
     if (tid == 0) {
@@ -728,76 +991,148 @@ __global__ void __launch_bounds__(T) sm_dense_kernel(DGeom g, const float2* __re
     }
     return;
   }
-  // a slot outside the windows was added to the spare slot: every thread
-  // reads the same value and takes the same branch
-  if (dense_fail || acc[nslots] != 0.f) {
-    if (tid == 0) {
-      row_nnz[blockIdx.x] = kRowToTable;
-      if (reasons) atomicAdd(reasons + 2, 1);
-    }
+  if (to_table) {
+    table(2);
     return;
   }
 
-  // Dense compaction layout: each warp takes a contiguous run of slots
-  // (slab-major, then U, then V).
-  constexpr int NW = T / 32;
-  const int lane = tid & 31, w = tid >> 5;
-  const int seg = ((nslots + NW - 1) / NW + 31) & ~31;
-  const int b0 = min(w * seg, nslots), b1 = min(b0 + seg, nslots);
-  auto voxel = [&](int slot, int* x, int* y, int* z) {
-    const int sa = slot / wuv;
-    const int rem = slot - sa * wuv;
-    const int u = rem / wv;
-    const int iu = ulo[sa] + u, iv = vlo[sa] + (rem - u * wv);
-    *x = A == 0 ? sa : iu;
+  // The groups' sums per voxel, and the cylinder test: stage[s * Wp + w] =
+  // the sum of a voxel of the row, 0 elsewhere.
+  const unsigned m_wv = div_magic(wv), m_na = div_magic(na), m_wp = div_magic(Wp), m_ks = div_magic(kSlabs);
+  auto voxel = [&](int s, int w, int* x, int* y, int* z) {
+    const int u = div_by(w, wv, m_wv);
+    const int iu = ulo[s] + u, iv = vlo[s] + (w - u * wv);
+    *x = A == 0 ? s : iu;
     *y = A == 0 ? iu : iv;
-    *z = A == 0 ? iv : sa;
+    *z = A == 0 ? iv : s;
   };
-  // First compaction pass: per warp, count the voxels with a positive sum
-  // that pass the cylinder test and clear the others.  A positive slot that
-  // decodes to a voxel outside the grid means the windows missed a voxel:
-  // the row goes to the table kernel.
-  {
-    int cnt = 0;
-    for (int b = b0; b < b1; b += 32) {
-      const int slot = b + lane;
-      bool keep = false;
-      if (slot < b1) {
-        const float v = acc[slot];
-        if (v > 0.f) {
-          int x, y, z;
-          voxel(slot, &x, &y, &z);
-          if (x < g.n[0] && y < g.n[1] && z < g.n[2]) {
-            keep = candidate_test(g, ch, x, y, z);
-          } else {
-            dense_fail = 1;
-          }
-          if (!keep) acc[slot] = 0.f;
+  for (int i = tid; i < na * Wp; i += T) {
+    const int w = div_by(i, na, m_na), s = i - w * na;
+    float v = 0.f;
+    if (w < W) {
+      const int t = div_by(s, kSlabs, m_ks);
+      const float* a = acc + ((s - t * kSlabs) * W + w) * S + t;
+      for (int k = 0; k < G; k++) v += a[k * nt];
+      if (v > 0.f) {
+        int x, y, z;
+        voxel(s, w, &x, &y, &z);
+        if (x < g.n[0] && y < g.n[1] && z < g.n[2]) {
+          if (!candidate_test(g, ch, x, y, z)) v = 0.f;
+        } else {
+          outside = 1;
         }
       }
-      cnt += __popc(__ballot_sync(0xffffffffu, keep));
     }
-    if (lane == 0) warp_sums[w] = cnt;
+    stage[s * Wp + w] = v;
   }
   __syncthreads();
-  if (dense_fail) {
-    if (tid == 0) {
-      row_nnz[blockIdx.x] = kRowToTable;
-      if (reasons) atomicAdd(reasons + 3, 1);
-    }
+  if (outside) {
+    table(3);
     return;
   }
-  // Second pass: after a scan of the warp counts, each warp writes its
-  // voxels in slot order -- column order for x slabs; z slabs are sorted
-  // below.
   const float fr = float(nrays);
-  const size_t base = size_t(blockIdx.x) * H;
-  int before = 0, total = 0;
-  for (int k = 0; k < NW; k++) {
-    const int c = warp_sums[k];
-    before += k < w ? c : 0;
-    total += c;
+  const size_t out = size_t(blockIdx.x) * H;
+  const int nz = g.n[2], nyz = g.n[1] * nz, n_out = na * Wp;
+  if (A == 0) {
+    // x slabs: slab-major, then y, z is column order; each warp takes a
+    // contiguous run of slots, counts its voxels, and after a scan of the
+    // counts writes them
+    const int seg = ((n_out + NW - 1) / NW + 31) & ~31;
+    const int b0 = min(warp * seg, n_out), b1 = min(b0 + seg, n_out);
+    int cnt = 0;
+    for (int b = b0 + lane; b - lane < b1; b += 32)
+      cnt += __popc(__ballot_sync(0xffffffffu, b < b1 && stage[b] > 0.f));
+    if (lane == 0) warp_sums[warp] = cnt;
+    __syncthreads();
+    int before = 0, total = 0;
+    for (int k = 0; k < NW; k++) {
+      before += k < warp ? warp_sums[k] : 0;
+      total += warp_sums[k];
+    }
+    if (total > H) {
+      if (tid == 0) {
+        row_nnz[blockIdx.x] = -1;
+        atomicOr(flags, 1);
+      }
+      return;
+    }
+    for (int b = b0 + lane; b - lane < b1; b += 32) {
+      const float v = b < b1 ? stage[b] : 0.f;
+      const unsigned m = __ballot_sync(0xffffffffu, v > 0.f);
+      if (v > 0.f) {
+        const int pos = before + __popc(m & ((1u << lane) - 1u));
+        int x, y, z;
+        const int s = div_by(b, Wp, m_wp);
+        voxel(s, b - s * Wp, &x, &y, &z);
+        st_col[out + pos] = x * nyz + y * nz + z;
+        st_val[out + pos] = RFDIV(v, fr);
+      }
+      before += __popc(m);
+    }
+    if (tid == 0) row_nnz[blockIdx.x] = total;
+    return;
   }
+  // z slabs: column order is (x, y, z).  Per (x, y) of the box that holds
+  // every slab's window, a bitmask of the z of the row's voxels; a voxel's
+  // place is the number of bits of the (x, y) before its own and of the z
+  // below its own.
+  for (int s = tid; s < na; s += T) {
+    atomicMin(&zbox[0], int(ulo[s]));
+    atomicMax(&zbox[1], int(ulo[s]) + wu);
+    atomicMin(&zbox[2], int(vlo[s]));
+    atomicMax(&zbox[3], int(vlo[s]) + wv);
+  }
+  __syncthreads();
+  const int x0 = zbox[0], y0 = zbox[2], wy = zbox[3] - y0;
+  const int nkeys = (zbox[1] - x0) * wy, words = (nz + 31) >> 5;
+  if ((long long)nkeys * (words + 1) > (long long)acc_floats) {
+    table(1);
+    return;
+  }
+  unsigned* mask = reinterpret_cast<unsigned*>(acc);   // [word][key]
+  int* first = reinterpret_cast<int*>(acc) + words * nkeys;
+  for (int i = tid; i < nkeys * words; i += T) mask[i] = 0u;
+  __syncthreads();
+  for (int i = tid; i < n_out; i += T)
+    if (stage[i] > 0.f) {
+      int x, y, z;
+      const int s = div_by(i, Wp, m_wp);
+      voxel(s, i - s * Wp, &x, &y, &z);
+      atomicOr(&mask[(z >> 5) * nkeys + (x - x0) * wy + (y - y0)], 1u << (z & 31));
+    }
+  __syncthreads();
+  int total = 0;
+  {
+    // exclusive scan of the keys' counts: each thread a run of keys
+    const int pk = (nkeys + T - 1) / T;
+    const int k0 = min(tid * pk, nkeys), k1 = min(k0 + pk, nkeys);
+    int run = 0;
+    for (int k = k0; k < k1; k++) {
+      int c = 0;
+      for (int w = 0; w < words; w++) c += __popc(mask[w * nkeys + k]);
+      first[k] = c;
+      run += c;
+    }
+    int incl = run;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    int off = incl - run;
+    for (int k = 0; k < NW; k++) {
+      off += k < warp ? warp_sums[k] : 0;
+      total += warp_sums[k];
+    }
+    for (int k = k0; k < k1; k++) {
+      const int c = first[k];
+      first[k] = off;
+      off += c;
+    }
+  }
+  __syncthreads();
   if (total > H) {
     if (tid == 0) {
       row_nnz[blockIdx.x] = -1;
@@ -805,105 +1140,18 @@ __global__ void __launch_bounds__(T) sm_dense_kernel(DGeom g, const float2* __re
     }
     return;
   }
-  for (int b = b0; b < b1; b += 32) {
-    const int slot = b + lane;
-    const bool keep = slot < b1 && acc[slot] > 0.f;
-    const unsigned m = __ballot_sync(0xffffffffu, keep);
-    if (keep) {
-      const int pos = before + __popc(m & ((1u << lane) - 1u));
+  for (int i = tid; i < n_out; i += T) {
+    const float v = stage[i];
+    if (v > 0.f) {
       int x, y, z;
-      voxel(slot, &x, &y, &z);
-      st_col[base + pos] = x * nyz + y * nz + z;
-      st_val[base + pos] = RFDIV(acc[slot], fr);
+      const int s = div_by(i, Wp, m_wp);
+      voxel(s, i - s * Wp, &x, &y, &z);
+      const int k = (x - x0) * wy + (y - y0), zw = z >> 5;
+      int pos = first[k] + __popc(mask[zw * nkeys + k] & ((1u << (z & 31)) - 1u));
+      for (int w = 0; w < zw; w++) pos += __popc(mask[w * nkeys + k]);
+      st_col[out + pos] = x * nyz + y * nz + z;
+      st_val[out + pos] = RFDIV(v, fr);
     }
-    before += __popc(m);
-  }
-  if (A == 0) {
-    if (tid == 0) row_nnz[blockIdx.x] = total;
-    return;
-  }
-  // z slabs: the entries ascend in z slab by slab, within a slab in (x, y).
-  // Column order is (x, y, z): a counting sort by (x, y) over the box that
-  // holds every slab's window places them, an entry's rank among the
-  // entries of its (x, y) being the number of their z below its own (a z
-  // bitmask per key).  When the box's counters do not fit beside the row's
-  // staging in shared memory (or the grid has more than 96 z planes), the
-  // bitonic sort does it.
-  __shared__ int zbox[4];
-  if (tid == 0) {
-    zbox[0] = INT_MAX;
-    zbox[1] = INT_MIN;
-    zbox[2] = INT_MAX;
-    zbox[3] = INT_MIN;
-  }
-  __syncthreads();
-  for (int sl = tid; sl < na; sl += T) {
-    atomicMin(&zbox[0], ulo[sl]);
-    atomicMax(&zbox[1], ulo[sl] + wu);
-    atomicMin(&zbox[2], vlo[sl]);
-    atomicMax(&zbox[3], vlo[sl] + wv);
-  }
-  for (int i = tid; i < total; i += T) {
-    keys[i] = st_col[base + i];
-    vals[i] = st_val[base + i];
-  }
-  __syncthreads();
-  const int wy = zbox[3] - zbox[2];
-  const int nkeys = (zbox[1] - zbox[0]) * wy;
-  constexpr int kKeyBytes = 16;  // counter + 96-bit z mask
-  const int key_cap = int((row_smem_bytes(H) - size_t(H) * 8) / kKeyBytes);
-  if (nkeys > key_cap || nz > 96) {
-    sort_and_write<T>(keys, vals, total, st_col, st_val, base, row_nnz + blockIdx.x);
-    return;
-  }
-  int* cnt = reinterpret_cast<int*>(smem + size_t(H) * 8);
-  unsigned* zmask = reinterpret_cast<unsigned*>(cnt + nkeys);
-  for (int i = tid; i < nkeys * 4; i += T) cnt[i] = 0;  // counters and masks
-  __syncthreads();
-  const int x0 = zbox[0], y0 = zbox[2];
-  for (int i = tid; i < total; i += T) {
-    const int c = keys[i];
-    const int x = c / nyz, r = c - x * nyz, y = r / nz, z = r - y * nz;
-    const int k = (x - x0) * wy + (y - y0);
-    atomicAdd(&cnt[k], 1);
-    atomicOr(&zmask[3 * k + (z >> 5)], 1u << (z & 31));
-  }
-  __syncthreads();
-  // exclusive scan of the counters: each thread a run of consecutive keys
-  {
-    const int per = (nkeys + T - 1) / T;
-    const int k0 = min(tid * per, nkeys), k1 = min(k0 + per, nkeys);
-    int run = 0;
-    for (int k = k0; k < k1; k++) run += cnt[k];
-    int incl = run;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    if (lane == 31) warp_sums[w] = incl;
-    __syncthreads();
-    int wbase = 0;
-    for (int q = 0; q < w; q++) wbase += warp_sums[q];
-    int off = wbase + incl - run;
-    for (int k = k0; k < k1; k++) {
-      const int c = cnt[k];
-      cnt[k] = off;
-      off += c;
-    }
-  }
-  __syncthreads();
-  for (int i = tid; i < total; i += T) {
-    const int c = keys[i];
-    const int x = c / nyz, r = c - x * nyz, y = r / nz, z = r - y * nz;
-    const int k = (x - x0) * wy + (y - y0);
-    const unsigned* m = zmask + 3 * k;
-    const int zw = z >> 5;
-    int rank = __popc(m[zw] & ((1u << (z & 31)) - 1u));
-    if (zw > 0) rank += __popc(m[0]);
-    if (zw > 1) rank += __popc(m[1]);
-    st_col[base + cnt[k] + rank] = c;
-    st_val[base + cnt[k] + rank] = vals[i];
   }
   if (tid == 0) row_nnz[blockIdx.x] = total;
 }
@@ -912,7 +1160,7 @@ __global__ void __launch_bounds__(T) sm_dense_kernel(DGeom g, const float2* __re
 // an open-addressing hash table of H keys in shared memory, then the voxels
 // with a positive sum that pass the cylinder test sorted into column order.
 // Each CTA takes rows blockIdx.x, blockIdx.x + gridDim.x, ... of the nrows.
-// With only_flagged it builds only the rows the dense kernel left with
+// With only_flagged it builds only the rows the slab kernel left with
 // kRowToTable and leaves the others alone (launched then with a small grid:
 // most workloads leave none, and the blocks only read the row states).
 template <int H, int T, bool OISO>
@@ -926,8 +1174,13 @@ __global__ void __launch_bounds__(T) sm_table_kernel(DGeom g, const float2* __re
   int* keys = reinterpret_cast<int*>(smem);
   float* vals = reinterpret_cast<float*>(smem + H * sizeof(int));
   __shared__ Channel ch;
-  __shared__ int overflow, bad_walk;
+  __shared__ int overflow, bad_walk, n_parallel;
   __shared__ int warp_sums[32];
+  // rays parallel to the planes of an axis: all candidates along that axis
+  // get their lengths, which the block's threads share (one thread alone
+  // takes 2-4 ms for one such ray, and a build of 20,000 rows meets about one)
+  constexpr int kMaxParallel = 256;
+  __shared__ int parallel[kMaxParallel];
 
   const int tid = threadIdx.x;
   const int nyz = g.n[1] * g.n[2];
@@ -948,6 +1201,7 @@ __global__ void __launch_bounds__(T) sm_table_kernel(DGeom g, const float2* __re
       channel_setup(g, sincos, cnl, ch);
       overflow = 0;
       bad_walk = 0;
+      n_parallel = 0;
     }
     for (int i = tid; i < H; i += T) {
       keys[i] = -1;
@@ -959,8 +1213,7 @@ __global__ void __launch_bounds__(T) sm_table_kernel(DGeom g, const float2* __re
       KeyIndex<H> kix{&table, nyz, nz};
       auto emit = [&](int ix, int iy, int iz, float L) { table.add(ix * nyz + iy * nz + iz, L); };
       const int part = int(__brev(threadIdx.x) >> 24);
-      for (int ray = tid; ray < nrays; ray += T) {
-        float r[6];
+      auto ray_ends = [&](int ray, float r[6]) {
         if (rays) {
           const float* src = rays + (li * int64_t(nrays) + ray) * 6;
 #pragma unroll
@@ -968,7 +1221,25 @@ __global__ void __launch_bounds__(T) sm_table_kernel(DGeom g, const float2* __re
         } else {
           make_ray(ch, seed, cnl, ray, r);
         }
-        walk_ray<OISO, 1>(g, ch, r, part, emit, kix, &bad_walk);
+      };
+      for (int ray = tid; ray < nrays; ray += T) {
+        float r[6];
+        ray_ends(ray, r);
+        if (r[0] == r[3] || r[1] == r[4] || r[2] == r[5]) {
+          const int at = atomicAdd(&n_parallel, 1);
+          if (at < kMaxParallel) {
+            parallel[at] = ray;
+            continue;
+          }
+        }
+        walk_ray<OISO>(g, ch, r, part, emit, kix, &bad_walk, 0, 1);
+      }
+      __syncthreads();
+      const int np = min(n_parallel, kMaxParallel);
+      for (int i = 0; i < np; i++) {
+        float r[6];
+        ray_ends(parallel[i], r);
+        walk_ray<OISO>(g, ch, r, 0, emit, kix, &bad_walk, tid, T);
       }
     }
     __syncthreads();
@@ -1022,6 +1293,37 @@ struct Level {
 constexpr Level kLevels[] = {{2048, 128}, {4096, 256}, {8192, 256}, {16384, 512}};
 constexpr int kNumLevels = 4;
 
+// Threads and shared memory of the slab kernel on a grid.  192 threads and
+// three blocks per SM for 2 mm voxels: the sums, kSlabs * W slots per thread,
+// are what fills shared memory.  W is the window of the 4x4x20 mm crystals
+// seen from any angle at the grid's pitch (16-24 slots for 75 % of the
+// channels at 2 mm, 20-30 at 1.5 mm); a row with a larger one runs with fewer
+// groups.  60,000 rows of 70^3 x 1000 rays / 12,345 of 100^3 x 999: 13.45 /
+// 4.76 ms; with 96 threads 13.9 / 6.4, 256: 15.1 / 4.8, 288: 15.2 / 5.9; with
+// room for four blocks (W = 16-18) 14.5-16.4 / 6.2-6.9, with two slabs per
+// thread 15.0 / 4.8, with one 17.3 / 5.9.
+SlabShape slab_shape(const DGeom& g) {
+  SlabShape sh;
+  // the most threads whose groups leave few of them idle
+  double best = 0.0;
+  for (int T = kSlabThreads; T >= 128; T -= 32) {
+    double used = 0.0;
+    for (int a = 0; a < 3; a += 2) {
+      const int nt = (g.n[a] + kSlabs - 1) / kSlabs;
+      if (g.n[a] <= kMaxSlabs && nt <= T) used += double(T / nt * nt) / T;
+    }
+    if (sh.threads == 0 || used > 1.1 * best) {
+      best = used;
+      sh.threads = T;
+    }
+  }
+  const double wy = g.segy / g.d[1] + 2.1, wh = 1.5 * g.segz / std::min(g.d[0], g.d[2]) + 2.1;
+  const int W = int(std::min(std::ceil(wy * wh), 64.0));
+  sh.acc_floats = (kSlabs * W + 3) * sh.threads;
+  sh.stage_floats = std::max(kSlabBatch * int(sizeof(SlabRay) / 4), std::min(50 * std::max(g.n[0], g.n[2]), 8192));
+  return sh;
+}
+
 template <int H, int T>
 cudaError_t launch_level(const DGeom& g, const float2* d_sincos, const int32_t* d_cnl, int64_t row0, int64_t nrows,
                          int nrays, uint32_t seed, const float* d_rays, int32_t* st_col, float* st_val,
@@ -1041,16 +1343,16 @@ cudaError_t launch_level(const DGeom& g, const float2* d_sincos, const int32_t* 
     return cudaGetLastError();
   }
   if (parts & 1) {
-    auto dense = oiso ? sm_dense_kernel<H, T, true> : sm_dense_kernel<H, T, false>;
-    const size_t dense_smem = row_smem_bytes(H);
-    e = cudaFuncSetAttribute(dense, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dense_smem));
+    const SlabShape sh = slab_shape(g);
+    e = cudaFuncSetAttribute(sm_slab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sh.smem()));
     if (e != cudaSuccess) return e;
-    dense<<<unsigned(nrows), T, dense_smem, s>>>(g, d_sincos, d_cnl, row0, nrays, seed, st_col, st_val, row_nnz,
-                                                 d_flags, d_reasons);
+    sm_slab_kernel<<<unsigned(nrows), unsigned(sh.threads), sh.smem(), s>>>(
+        g, d_sincos, d_cnl, row0, nrays, seed, H, sh.acc_floats, sh.stage_floats, st_col, st_val, row_nnz, d_flags,
+        d_reasons);
     note_launches(1);
   }
   if (parts & 2) {
-    // the rows the dense kernel left to the table (a few per million on
+    // the rows the slab kernel left to the table (a few per million on
     // the centred-cube workloads), four blocks per SM looking through the
     // row states
     const int64_t tb = std::min<int64_t>(nrows, 148 * 4);
