@@ -224,15 +224,28 @@ __device__ __forceinline__ void make_ray(const Channel& ch, uint32_t seed, int c
 }
 
 // The warp's next work item: lane 0 draws it from the counter at `next`
-// and broadcasts it.  Called by all 32 lanes together.  The row passes draw
-// kRowChunk rows at a time: one draw per row (5.14M draws on one address)
-// makes the forward pass twice as slow, one per 16 rows takes 7 % off the
-// grid stride's time.
-constexpr int kRowChunk = 16;
+// and broadcasts it.  Called by all 32 lanes together.  Draws from one
+// address are served one after the other, ~1.5 ns each (343,000 draws of one
+// short column each took 0.5 ms of a back pass that moves its bytes in 0.2),
+// so an item is several rows or columns.
+constexpr int kDrawWarps = 148 * 40;  // warps that draw
 __device__ __forceinline__ int64_t warp_next(unsigned long long* next, int lane) {
   unsigned long long q = 0;
   if (lane == 0) q = atomicAdd(next, 1ull);
   return int64_t(__shfl_sync(0xffffffffu, q, 0));
+}
+
+// Below this many rows (eight to a warp) the row passes take them by a grid
+// stride, since the draws would take longer than the rows (28,561 rows of 438
+// entries: 47 us drawn, 31 us strided; 57,122 of 1535: 157 drawn, 164 strided).
+constexpr int64_t kDrawRows = int64_t(kDrawWarps) * 8;
+
+// Rows a draw takes: 16 (one draw per row makes the forward pass of 5.14M rows
+// twice as slow, one per 16 takes 7 % off the grid stride's time), fewer where
+// that would leave less than eight draws to a warp (200,000 rows: 4).
+__device__ __forceinline__ int draw_rows(int64_t m) {
+  const int64_t c = m / (int64_t(kDrawWarps) * 8);
+  return int(c < 1 ? 1 : (c > 16 ? 16 : c));
 }
 
 }  // namespace raptr

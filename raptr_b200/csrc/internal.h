@@ -282,7 +282,7 @@ cudaError_t launch_transpose_blocked(int64_t m, int64_t n, int B, const int64_t*
                                      float* tval, cudaStream_t s);
 // e_i = y_i / (A x)_i (0 for y_i == 0); optional FP64 log-likelihood sums.
 // With `next` (an 8-byte counter, zero at launch) the warps draw rows from
-// it, kRowChunk at a time.
+// it, a few at a time.
 cudaError_t launch_mlem_forward(int64_t m, const int64_t* rp, const int32_t* col, const float* val, const float* y,
                                 const float* x, const int32_t* rank, float* e, double* d_ll, cudaStream_t s,
                                 unsigned long long* next = nullptr);

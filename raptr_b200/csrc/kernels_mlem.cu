@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "columns.cuh"
 #include "internal.h"
 
 namespace raptr {
@@ -16,10 +17,11 @@ namespace raptr {
 namespace {
 
 constexpr int kThreads = 256;
-// CTAs per SM the FP32 MLEM passes are compiled for: 5 (48 registers) runs
-// them 2-4 % faster than the 4 their unbounded register use (60-62) allows;
-// 6 (40 registers, with spills) is slower.
-constexpr int kPassBlocks = 5;
+// CTAs per SM the FP32 MLEM passes are compiled for.  The forward pass with 5
+// (48 registers) is 2-4 % faster than the 4 its unbounded register use (60)
+// allows; 6 (40 registers, with spills) is slower.  The back pass spills at 48
+// registers (281 against 226 us on 70^3 x 200,000 rows) and takes 4.
+constexpr int kPassBlocks = 5, kBackBlocks = 4;
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -60,7 +62,6 @@ __device__ __forceinline__ float row_dot(const int32_t* __restrict__ col, const 
   }
   int64_t a = (b + 3) & ~int64_t(3);
   if (a > e) a = e;
-  if (b + lane < a) acc += __ldg(val + b + lane) * __ldg(x + __ldg(col + b + lane));
   const int64_t nq = (e - a) >> 2;
   const int4* c4 = reinterpret_cast<const int4*>(col + a);
   const float4* v4 = reinterpret_cast<const float4*>(val + a);
@@ -80,13 +81,22 @@ __device__ __forceinline__ float row_dot(const int32_t* __restrict__ col, const 
     acc2 += w2.x * g20 + w2.y * g21 + w2.z * g22 + w2.w * g23;
     acc3 += w3.x * g30 + w3.y * g31 + w3.z * g32 + w3.w * g33;
   }
-  for (; q < nq; q += 32) {
-    const int4 c0 = __ldg(c4 + q);
-    const float4 w0 = __ldg(v4 + q);
-    acc += w0.x * __ldg(x + c0.x) + w0.y * __ldg(x + c0.y) + w0.z * __ldg(x + c0.z) + w0.w * __ldg(x + c0.w);
+  // The rest in steps of two quads per lane with predicated loads, the entries
+  // before the first and after the last whole quad along with the first of them.
+  const int64_t t = lane < 16 ? b + lane : a + (nq << 2) + (lane - 16);
+  const bool edge = lane < 16 ? t < a : t < e;
+  const int ct = edge ? __ldg(col + t) : 0;
+  const float wt = edge ? __ldg(val + t) : 0.f;
+  for (; q - lane < nq; q += 64) {
+    const bool in0 = q < nq, in1 = q + 32 < nq;
+    const int4 c0 = in0 ? __ldg(c4 + q) : make_int4(0, 0, 0, 0);
+    const int4 c1 = in1 ? __ldg(c4 + q + 32) : make_int4(0, 0, 0, 0);
+    const float4 w0 = in0 ? __ldg(v4 + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 w1 = in1 ? __ldg(v4 + q + 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (in0) acc += w0.x * __ldg(x + c0.x) + w0.y * __ldg(x + c0.y) + w0.z * __ldg(x + c0.z) + w0.w * __ldg(x + c0.w);
+    if (in1) acc1 += w1.x * __ldg(x + c1.x) + w1.y * __ldg(x + c1.y) + w1.z * __ldg(x + c1.z) + w1.w * __ldg(x + c1.w);
   }
-  const int64_t t = a + (nq << 2) + lane;
-  if (t < e) acc += __ldg(val + t) * __ldg(x + __ldg(col + t));
+  if (edge) acc2 += wt * __ldg(x + ct);
   return warp_sum((acc + acc1) + (acc2 + acc3));
 }
 
@@ -500,11 +510,12 @@ __global__ void __launch_bounds__(kThreads, kPassBlocks) mlem_forward_kernel(int
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
   double ly = 0.0, lt = 0.0;
-  // rows [r0, r1): kRowChunk rows drawn from the counter at `next`, or one
-  // row by a grid stride
-  int64_t r0 = next ? warp_next(next, lane) * kRowChunk : (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  for (; r0 < m; r0 = next ? warp_next(next, lane) * kRowChunk : r0 + nw)
-  for (int64_t r = r0, r1 = next ? min(r0 + kRowChunk, m) : r0 + 1; r < r1; r++) {
+  // rows [r0, r1): a few rows drawn from the counter at `next`, or one row by
+  // a grid stride
+  const int chunk = draw_rows(m);
+  int64_t r0 = next ? warp_next(next, lane) * chunk : (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  for (; r0 < m; r0 = next ? warp_next(next, lane) * chunk : r0 + nw)
+  for (int64_t r = r0, r1 = next ? min(r0 + chunk, m) : r0 + 1; r < r1; r++) {
     const float yi = __ldg(y + r);
     const int64_t dst = rank ? int64_t(__ldg(rank + r)) : r;
     if (yi == 0.f) {
@@ -530,14 +541,11 @@ __global__ void __launch_bounds__(kThreads, kPassBlocks) mlem_forward_kernel(int
 // Back projection by columns: c_j = <column j of A, e>.  With UPDATE the
 // MLEM update follows in the epilogue: xx_j = x_j*c_j/(s_j + (s_j==0)) and
 // acc += sum xx (FP64); without it c_j is stored.  With a column counter
-// (`next`, zero at launch) each warp draws its next column from it, so that
-// warps whose columns were short take more of them: columns run from a few
-// entries at the edge of the field of view to ~10^4 at its centre, and a
+// (`next`, zero at launch) the warps draw columns from it (back_columns): a
 // grid stride leaves the kernel waiting on the warps that drew the longest
-// (0.85 instead of 0.72 of HBM on the 70^3 x 5.14M matrix).  Without it the
-// columns go by a grid stride.
+// (0.85 instead of 0.72 of HBM on the 70^3 x 5.14M matrix).
 template <bool VEC, bool UPDATE>
-__global__ void __launch_bounds__(kThreads, kPassBlocks) mlem_back_kernel(int64_t n, const int64_t* __restrict__ cp,
+__global__ void __launch_bounds__(kThreads, kBackBlocks) mlem_back_kernel(int64_t n, const int64_t* __restrict__ cp,
                                                              const int32_t* __restrict__ trow,
                                                              const float* __restrict__ tval,
                                                              const float* __restrict__ e,
@@ -545,23 +553,11 @@ __global__ void __launch_bounds__(kThreads, kPassBlocks) mlem_back_kernel(int64_
                                                              const float* __restrict__ sens, float* __restrict__ out,
                                                              double* __restrict__ acc, unsigned long long* next) {
   const int lane = threadIdx.x & 31;
-  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  double sum = 0.0;
-  int64_t j = next ? warp_next(next, lane) : (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  for (; j < n; j = next ? warp_next(next, lane) : j + nw) {
-    const float c = row_dot<VEC>(trow, tval, cp[j], cp[j + 1], e, lane);
-    if (lane == 0) {
-      if (UPDATE) {
-        float dvs = sens[j];
-        dvs += float(dvs == 0.f);
-        const float xx = __fdiv_rn(__fmul_rn(x[j], c), dvs);
-        out[j] = xx;
-        sum += double(xx);
-      } else {
-        out[j] = c;
-      }
-    }
-  }
+  const double sum = back_columns<UPDATE>(
+      n, cp, x, sens, out, next, [&](int64_t b, int64_t b1) { return row_dot<VEC>(trow, tval, b, b1, e, lane); },
+      [&](const int64_t(&b)[4], const int(&len)[4]) {
+        return short_columns(trow, tval, b, len, e, lane, [](float v) { return v; });
+      });
   if (UPDATE) block_add_double(sum, acc);
 }
 
@@ -770,6 +766,7 @@ cudaError_t launch_mlem_forward(int64_t m, const int64_t* rp, const int32_t* col
                                 const float* x, const int32_t* rank, float* e, double* d_ll, cudaStream_t s,
                                 unsigned long long* next) {
   if (m > 0) {
+    if (m < kDrawRows) next = nullptr;
     mlem_forward_kernel<<<row_grid(m), kThreads, 0, s>>>(m, rp, col, val, y, x, rank, e, d_ll, next);
     note_launches(1);
   }

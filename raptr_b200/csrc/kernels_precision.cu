@@ -16,6 +16,7 @@
 
 #include <cuda_fp16.h>
 
+#include "columns.cuh"
 #include "internal.h"
 
 namespace raptr {
@@ -166,10 +167,11 @@ __global__ void __launch_bounds__(kThreads) mlem_forward_half_kernel(
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
   double ly = 0.0, lt = 0.0;
-  // rows drawn kRowChunk at a time from `next` when given, as the FP32 pass
-  int64_t r0 = next ? warp_next(next, lane) * kRowChunk : (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  for (; r0 < m; r0 = next ? warp_next(next, lane) * kRowChunk : r0 + nw)
-  for (int64_t r = r0, r1 = next ? min(r0 + kRowChunk, m) : r0 + 1; r < r1; r++) {
+  // rows drawn a few at a time from `next` when given, as the FP32 pass
+  const int chunk = draw_rows(m);
+  int64_t r0 = next ? warp_next(next, lane) * chunk : (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  for (; r0 < m; r0 = next ? warp_next(next, lane) * chunk : r0 + nw)
+  for (int64_t r = r0, r1 = next ? min(r0 + chunk, m) : r0 + 1; r < r1; r++) {
     const float yi = __ldg(y + r);
     const int64_t dst = rank ? int64_t(__ldg(rank + r)) : r;
     if (yi == 0.f) {
@@ -203,7 +205,6 @@ __device__ __forceinline__ float col_dot_half(const int32_t* __restrict__ trow, 
   float s = 0.f, c = 0.f;
   int64_t a = (b + 3) & ~int64_t(3);
   if (a > e) a = e;
-  if (b + lane < a) two_sum_add(s, c, h2f(hv[b + lane]) * __ldg(ev + __ldg(trow + b + lane)));
   const int64_t nq = (e - a) >> 2;
   const int4* t4 = reinterpret_cast<const int4*>(trow + a);
   const uint2* h4 = reinterpret_cast<const uint2*>(hv + a);
@@ -228,28 +229,36 @@ __device__ __forceinline__ float col_dot_half(const int32_t* __restrict__ trow, 
     two_sum_add(s, c, (f4.x * g8 + f4.y * g9) + (f5.x * g10 + f5.y * g11));
     two_sum_add(s, c, (f6.x * g12 + f6.y * g13) + (f7.x * g14 + f7.y * g15));
   }
-  for (; q + 32 < nq; q += 64) {
-    const int4 r0 = __ldcs(t4 + q), r1 = __ldcs(t4 + q + 32);
-    const uint2 w0 = __ldcs(h4 + q), w1 = __ldcs(h4 + q + 32);
-    const float g0 = __ldg(ev + r0.x), g1 = __ldg(ev + r0.y), g2 = __ldg(ev + r0.z), g3 = __ldg(ev + r0.w);
-    const float g4 = __ldg(ev + r1.x), g5 = __ldg(ev + r1.y), g6 = __ldg(ev + r1.z), g7 = __ldg(ev + r1.w);
-    const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&w0.x));
-    const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&w0.y));
-    const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&w1.x));
-    const float2 f3 = __half22float2(*reinterpret_cast<const __half2*>(&w1.y));
-    two_sum_add(s, c, (f0.x * g0 + f0.y * g1) + (f1.x * g2 + f1.y * g3));
-    two_sum_add(s, c, (f2.x * g4 + f2.y * g5) + (f3.x * g6 + f3.y * g7));
+  // the rest as one step with predicated loads (see the FP32 row_dot)
+  int4 r[4];
+  uint2 w[4];
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    const bool in = q + 32 * u < nq;
+    r[u] = in ? __ldcs(t4 + q + 32 * u) : make_int4(0, 0, 0, 0);
+    w[u] = in ? __ldcs(h4 + q + 32 * u) : make_uint2(0u, 0u);
   }
-  for (; q < nq; q += 32) {
-    const int4 r0 = __ldcs(t4 + q);
-    const uint2 w0 = __ldcs(h4 + q);
-    const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&w0.x));
-    const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&w0.y));
-    two_sum_add(s, c, (f0.x * __ldg(ev + r0.x) + f0.y * __ldg(ev + r0.y)) +
-                          (f1.x * __ldg(ev + r0.z) + f1.y * __ldg(ev + r0.w)));
+  const int64_t t = lane < 16 ? b + lane : a + (nq << 2) + (lane - 16);
+  const bool edge = lane < 16 ? t < a : t < e;
+  const int rt = edge ? __ldg(trow + t) : 0;
+  const float wt = edge ? h2f(hv[t]) : 0.f;
+  float g[4][4];
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    const bool in = q + 32 * u < nq;
+    g[u][0] = in ? __ldg(ev + r[u].x) : 0.f;
+    g[u][1] = in ? __ldg(ev + r[u].y) : 0.f;
+    g[u][2] = in ? __ldg(ev + r[u].z) : 0.f;
+    g[u][3] = in ? __ldg(ev + r[u].w) : 0.f;
   }
-  const int64_t t = a + (nq << 2) + lane;
-  if (t < e) two_sum_add(s, c, h2f(hv[t]) * __ldg(ev + __ldg(trow + t)));
+  const float gt = edge ? __ldg(ev + rt) : 0.f;
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&w[u].x));
+    const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&w[u].y));
+    two_sum_add(s, c, (f0.x * g[u][0] + f0.y * g[u][1]) + (f1.x * g[u][2] + f1.y * g[u][3]));
+  }
+  two_sum_add(s, c, wt * gt);
   // combine the lanes' (sum, compensation) pairs, compensated too
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -261,10 +270,9 @@ __device__ __forceinline__ float col_dot_half(const int32_t* __restrict__ trow, 
   return s + c;
 }
 
-// Columns are drawn from the counter at `next` when it is given (see
-// mlem_back_kernel), else taken by a grid stride.
+// Columns as in mlem_back_kernel (back_columns).
 template <bool UPDATE>
-__global__ void __launch_bounds__(kThreads) mlem_back_half_kernel(int64_t n, const int64_t* __restrict__ cp,
+__global__ void __launch_bounds__(kThreads, 4) mlem_back_half_kernel(int64_t n, const int64_t* __restrict__ cp,
                                                                   const int32_t* __restrict__ trow,
                                                                   const uint16_t* __restrict__ htval,
                                                                   const float* __restrict__ e,
@@ -273,23 +281,12 @@ __global__ void __launch_bounds__(kThreads) mlem_back_half_kernel(int64_t n, con
                                                                   float* __restrict__ out, double* __restrict__ acc,
                                                                   unsigned long long* next) {
   const int lane = threadIdx.x & 31;
-  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  double sum = 0.0;
-  int64_t j = next ? warp_next(next, lane) : (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  for (; j < n; j = next ? warp_next(next, lane) : j + nw) {
-    const float c = col_dot_half(trow, htval, cp[j], cp[j + 1], e, lane);
-    if (lane == 0) {
-      if (UPDATE) {
-        float dvs = sens[j];
-        dvs += float(dvs == 0.f);
-        const float xx = __fdiv_rn(__fmul_rn(x[j], c), dvs);
-        out[j] = xx;
-        sum += double(xx);
-      } else {
-        out[j] = c;
-      }
-    }
-  }
+  const double sum = back_columns<UPDATE>(
+      n, cp, x, sens, out, next, [&](int64_t b, int64_t b1) { return col_dot_half(trow, htval, b, b1, e, lane); },
+      [&](const int64_t(&b)[4], const int(&len)[4]) {
+        return short_columns(trow, reinterpret_cast<const unsigned short*>(htval), b, len, e, lane,
+                             [](unsigned short v) { return h2f(v); });
+      });
   if (UPDATE) block_add_d(sum, acc);
 }
 
@@ -561,15 +558,16 @@ __device__ __forceinline__ float packed_col_dot(const uint4* __restrict__ w, int
 }
 
 // The FP16 forward pass over delta-coded rows: e'[rank_i] = rscale_i * y_i /
-// (A x)_i, rows drawn kRowChunk at a time from `next` (zero at launch).
+// (A x)_i, rows drawn a few at a time from `next` (zero at launch).
 __global__ void __launch_bounds__(kThreads) mlem_forward_packed_kernel(
     int64_t m, const int64_t* __restrict__ seg, const int32_t* __restrict__ anchor, const uint4* __restrict__ words,
     const float* __restrict__ rscale, const float* __restrict__ y, const float* __restrict__ x,
     const int32_t* __restrict__ rank, float* __restrict__ e, double* __restrict__ ll, unsigned long long* next) {
   const int lane = threadIdx.x & 31;
   double ly = 0.0, lt = 0.0;
-  for (int64_t r0 = warp_next(next, lane) * kRowChunk; r0 < m; r0 = warp_next(next, lane) * kRowChunk)
-    for (int64_t r = r0, r1 = min(r0 + kRowChunk, m); r < r1; r++) {
+  const int chunk = draw_rows(m);
+  for (int64_t r0 = warp_next(next, lane) * chunk; r0 < m; r0 = warp_next(next, lane) * chunk)
+    for (int64_t r = r0, r1 = min(r0 + chunk, m); r < r1; r++) {
       const float yi = __ldg(y + r);
       const int64_t dst = rank ? int64_t(__ldg(rank + r)) : r;
       if (yi == 0.f) {
@@ -648,6 +646,7 @@ cudaError_t launch_mlem_forward_half(int64_t m, const int64_t* rp, const int32_t
                                      const float* rscale, const float* y, const float* x, const int32_t* rank,
                                      float* e, double* d_ll, cudaStream_t s, unsigned long long* next) {
   if (m <= 0) return cudaSuccess;
+  if (m < kDrawRows) next = nullptr;
   mlem_forward_half_kernel<<<grid_rows(m), kThreads, 0, s>>>(m, rp, col, hval, rscale, y, x, rank, e, d_ll, next);
   note_launches(1);
   return cudaGetLastError();
