@@ -49,64 +49,13 @@ __device__ __forceinline__ void block_add_double(double v, double* dst) {
   }
 }
 
-// Dot product of CSR row [b, e) with x, computed by one warp; every lane
-// returns the sum.  Head and tail are scalar, the aligned body uses
-// 16-byte loads of four columns and four values per lane.
-template <bool VEC>
-__device__ __forceinline__ float row_dot(const int32_t* __restrict__ col, const float* __restrict__ val, int64_t b,
-                                         int64_t e, const float* __restrict__ x, int lane) {
-  float acc = 0.f;
-  if (!VEC) {
-    for (int64_t k = b + lane; k < e; k += 32) acc += __ldg(val + k) * __ldg(x + __ldg(col + k));
-    return warp_sum(acc);
-  }
-  int64_t a = (b + 3) & ~int64_t(3);
-  if (a > e) a = e;
-  const int64_t nq = (e - a) >> 2;
-  const int4* c4 = reinterpret_cast<const int4*>(col + a);
-  const float4* v4 = reinterpret_cast<const float4*>(val + a);
-  int64_t q = lane;
-  // Four quads (16 entries) per lane per step: 8 independent 16-byte loads,
-  // then 16 independent gathers, kept in flight together.
-  float acc1 = 0.f, acc2 = 0.f, acc3 = 0.f;
-  for (; q + 96 < nq; q += 128) {
-    const int4 c0 = __ldg(c4 + q), c1 = __ldg(c4 + q + 32), c2 = __ldg(c4 + q + 64), c3 = __ldg(c4 + q + 96);
-    const float4 w0 = __ldg(v4 + q), w1 = __ldg(v4 + q + 32), w2 = __ldg(v4 + q + 64), w3 = __ldg(v4 + q + 96);
-    const float g00 = __ldg(x + c0.x), g01 = __ldg(x + c0.y), g02 = __ldg(x + c0.z), g03 = __ldg(x + c0.w);
-    const float g10 = __ldg(x + c1.x), g11 = __ldg(x + c1.y), g12 = __ldg(x + c1.z), g13 = __ldg(x + c1.w);
-    const float g20 = __ldg(x + c2.x), g21 = __ldg(x + c2.y), g22 = __ldg(x + c2.z), g23 = __ldg(x + c2.w);
-    const float g30 = __ldg(x + c3.x), g31 = __ldg(x + c3.y), g32 = __ldg(x + c3.z), g33 = __ldg(x + c3.w);
-    acc += w0.x * g00 + w0.y * g01 + w0.z * g02 + w0.w * g03;
-    acc1 += w1.x * g10 + w1.y * g11 + w1.z * g12 + w1.w * g13;
-    acc2 += w2.x * g20 + w2.y * g21 + w2.z * g22 + w2.w * g23;
-    acc3 += w3.x * g30 + w3.y * g31 + w3.z * g32 + w3.w * g33;
-  }
-  // The rest in steps of two quads per lane with predicated loads, the entries
-  // before the first and after the last whole quad along with the first of them.
-  const int64_t t = lane < 16 ? b + lane : a + (nq << 2) + (lane - 16);
-  const bool edge = lane < 16 ? t < a : t < e;
-  const int ct = edge ? __ldg(col + t) : 0;
-  const float wt = edge ? __ldg(val + t) : 0.f;
-  for (; q - lane < nq; q += 64) {
-    const bool in0 = q < nq, in1 = q + 32 < nq;
-    const int4 c0 = in0 ? __ldg(c4 + q) : make_int4(0, 0, 0, 0);
-    const int4 c1 = in1 ? __ldg(c4 + q + 32) : make_int4(0, 0, 0, 0);
-    const float4 w0 = in0 ? __ldg(v4 + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 w1 = in1 ? __ldg(v4 + q + 32) : make_float4(0.f, 0.f, 0.f, 0.f);
-    if (in0) acc += w0.x * __ldg(x + c0.x) + w0.y * __ldg(x + c0.y) + w0.z * __ldg(x + c0.z) + w0.w * __ldg(x + c0.w);
-    if (in1) acc1 += w1.x * __ldg(x + c1.x) + w1.y * __ldg(x + c1.y) + w1.z * __ldg(x + c1.z) + w1.w * __ldg(x + c1.w);
-  }
-  if (edge) acc2 += wt * __ldg(x + ct);
-  return warp_sum((acc + acc1) + (acc2 + acc3));
-}
-
-// Dot product of CSR row [b, e) with x, one warp, lanes on consecutive
-// entries: each step loads U entries per lane (32*U consecutive entries per
+// The lane's part of the dot product of entries [b, e) with x, one warp, lanes
+// on consecutive entries: each step loads U entries per lane (32*U consecutive entries per
 // warp, coalesced, streamed past the caches) and then gathers x for all of
 // them; one gather instruction covers 32 neighbouring columns of the row,
 // which sit in few cache lines because a row's voxels are sorted.
 template <int U>
-__device__ __forceinline__ float row_dot_seq(const int32_t* __restrict__ col, const float* __restrict__ val, int64_t b,
+__device__ __forceinline__ float seq_part(const int32_t* __restrict__ col, const float* __restrict__ val, int64_t b,
                                              int64_t e, const float* __restrict__ x, int lane) {
   static_assert(U % 4 == 0, "U is a multiple of 4");
   float acc0 = 0.f, acc1 = 0.f, acc2 = 0.f, acc3 = 0.f;
@@ -130,7 +79,78 @@ __device__ __forceinline__ float row_dot_seq(const int32_t* __restrict__ col, co
   }
   if (k < e) {
     // the rest of the row (fewer than 32*U entries) as one more step with
-    // predicated loads, so that its loads are in flight together
+    // predicated loads, so that its loads are in flight together; x is read
+    // for entries only (its other elements may be infinite)
+    int c[U];
+    float v[U], g[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const bool in = k + 32 * u < e;
+      c[u] = in ? __ldcs(col + k + 32 * u) : -1;
+      v[u] = in ? __ldcs(val + k + 32 * u) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) g[u] = c[u] >= 0 ? __ldg(x + c[u]) : 0.f;
+#pragma unroll
+    for (int u = 0; u < U; u += 4) {
+      acc0 += v[u] * g[u];
+      acc1 += v[u + 1] * g[u + 1];
+      acc2 += v[u + 2] * g[u + 2];
+      acc3 += v[u + 3] * g[u + 3];
+    }
+  }
+  return (acc0 + acc1) + (acc2 + acc3);
+}
+
+// Dot product of CSR row [b, e) with x; every lane returns it.
+template <int U>
+__device__ __forceinline__ float row_dot_seq(const int32_t* __restrict__ col, const float* __restrict__ val, int64_t b,
+                                             int64_t e, const float* __restrict__ x, int lane) {
+  return warp_sum(seq_part<U>(col, val, b, e, x, lane));
+}
+
+
+// Dot product of a column [b, e) of the transpose with x (the ratios), by one
+// warp; every lane returns it.  Whole steps of 512 entries by 16-byte loads of
+// four indices and four values per lane (VEC: the arrays are 16-byte aligned),
+// the rest as seq_part, whose gathers fall into a quarter of the sectors: long
+// columns are 2-3 % faster with the former, those of a few hundred entries
+// 5-14 % with the latter.
+template <bool VEC>
+__device__ __forceinline__ float col_dot(const int32_t* __restrict__ col, const float* __restrict__ val, int64_t b,
+                                         int64_t e, const float* __restrict__ x, int lane) {
+  const int64_t a = (b + 3) & ~int64_t(3);
+  if (!VEC || e - a < 512) return row_dot_seq<8>(col, val, b, e, x, lane);
+  const int64_t steps = (e - a) >> 9;
+  const int4* c4 = reinterpret_cast<const int4*>(col + a) + lane;
+  const float4* v4 = reinterpret_cast<const float4*>(val + a) + lane;
+  float acc = 0.f, acc1 = 0.f, acc2 = 0.f, acc3 = 0.f;
+  if (b + lane < a) acc = __ldg(val + b + lane) * __ldg(x + __ldg(col + b + lane));
+  for (int64_t i = 0; i < steps; i++, c4 += 128, v4 += 128) {
+    const int4 c0 = __ldg(c4), c1 = __ldg(c4 + 32), c2 = __ldg(c4 + 64), c3 = __ldg(c4 + 96);
+    const float4 w0 = __ldg(v4), w1 = __ldg(v4 + 32), w2 = __ldg(v4 + 64), w3 = __ldg(v4 + 96);
+    const float g00 = __ldg(x + c0.x), g01 = __ldg(x + c0.y), g02 = __ldg(x + c0.z), g03 = __ldg(x + c0.w);
+    const float g10 = __ldg(x + c1.x), g11 = __ldg(x + c1.y), g12 = __ldg(x + c1.z), g13 = __ldg(x + c1.w);
+    const float g20 = __ldg(x + c2.x), g21 = __ldg(x + c2.y), g22 = __ldg(x + c2.z), g23 = __ldg(x + c2.w);
+    const float g30 = __ldg(x + c3.x), g31 = __ldg(x + c3.y), g32 = __ldg(x + c3.z), g33 = __ldg(x + c3.w);
+    acc += w0.x * g00 + w0.y * g01 + w0.z * g02 + w0.w * g03;
+    acc1 += w1.x * g10 + w1.y * g11 + w1.z * g12 + w1.w * g13;
+    acc2 += w2.x * g20 + w2.y * g21 + w2.z * g22 + w2.w * g23;
+    acc3 += w3.x * g30 + w3.y * g31 + w3.z * g32 + w3.w * g33;
+  }
+  acc += seq_part<8>(col, val, a + (steps << 9), e, x, lane);
+  return warp_sum((acc + acc1) + (acc2 + acc3));
+}
+
+// y[col] += f * val over CSR row [b, e), by one warp, lanes on consecutive
+// entries as in row_dot_seq: the 32 reductions of an instruction fall into ~10
+// sectors of L2, which takes them sector by sector (with four consecutive
+// entries per lane, 16-byte loads, they fell into ~30).  Streaming loads: this is
+// the last use of the row in the pass.
+template <int U>
+__device__ __forceinline__ void row_scatter(const int32_t* __restrict__ col, const float* __restrict__ val, int64_t b,
+                                            int64_t e, float f, float* __restrict__ y, int lane) {
+  for (int64_t k = b + lane; k - lane < e; k += 32 * U) {
     int c[U];
     float v[U];
 #pragma unroll
@@ -140,41 +160,9 @@ __device__ __forceinline__ float row_dot_seq(const int32_t* __restrict__ col, co
       v[u] = in ? __ldcs(val + k + 32 * u) : 0.f;
     }
 #pragma unroll
-    for (int u = 0; u < U; u += 4) {
-      acc0 += v[u] * __ldg(x + c[u]);
-      acc1 += v[u + 1] * __ldg(x + c[u + 1]);
-      acc2 += v[u + 2] * __ldg(x + c[u + 2]);
-      acc3 += v[u + 3] * __ldg(x + c[u + 3]);
-    }
+    for (int u = 0; u < U; u++)
+      if (k + 32 * u < e) atomicAdd(y + c[u], v[u] * f);
   }
-  return warp_sum((acc0 + acc1) + (acc2 + acc3));
-}
-
-// y[col] += f * val over CSR row [b, e), by one warp.  Streaming loads:
-// this is the last use of the row in the pass.
-template <bool VEC>
-__device__ __forceinline__ void row_scatter(const int32_t* __restrict__ col, const float* __restrict__ val, int64_t b,
-                                            int64_t e, float f, float* __restrict__ y, int lane) {
-  if (!VEC) {
-    for (int64_t k = b + lane; k < e; k += 32) atomicAdd(y + __ldcs(col + k), __ldcs(val + k) * f);
-    return;
-  }
-  int64_t a = (b + 3) & ~int64_t(3);
-  if (a > e) a = e;
-  if (b + lane < a) atomicAdd(y + __ldcs(col + b + lane), __ldcs(val + b + lane) * f);
-  const int64_t nq = (e - a) >> 2;
-  const int4* c4 = reinterpret_cast<const int4*>(col + a);
-  const float4* v4 = reinterpret_cast<const float4*>(val + a);
-  for (int64_t q = lane; q < nq; q += 32) {
-    int4 c = __ldcs(c4 + q);
-    float4 w = __ldcs(v4 + q);
-    atomicAdd(y + c.x, w.x * f);
-    atomicAdd(y + c.y, w.y * f);
-    atomicAdd(y + c.z, w.z * f);
-    atomicAdd(y + c.w, w.w * f);
-  }
-  const int64_t t = a + (nq << 2) + lane;
-  if (t < e) atomicAdd(y + __ldcs(col + t), __ldcs(val + t) * f);
 }
 
 __global__ void __launch_bounds__(kThreads) spmv_n_kernel(int64_t m, const int64_t* __restrict__ rp,
@@ -190,7 +178,6 @@ __global__ void __launch_bounds__(kThreads) spmv_n_kernel(int64_t m, const int64
   }
 }
 
-template <bool VEC>
 __global__ void __launch_bounds__(kThreads) spmv_t_kernel(int64_t m, const int64_t* __restrict__ rp,
                                                           const int32_t* __restrict__ col,
                                                           const float* __restrict__ val, float alpha,
@@ -199,7 +186,7 @@ __global__ void __launch_bounds__(kThreads) spmv_t_kernel(int64_t m, const int64
   const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
   for (int64_t r = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; r < m; r += nw) {
     float f = alpha * x[r];
-    if (f != 0.f) row_scatter<VEC>(col, val, rp[r], rp[r + 1], f, y, lane);
+    if (f != 0.f) row_scatter<8>(col, val, rp[r], rp[r + 1], f, y, lane);
   }
 }
 
@@ -294,7 +281,6 @@ __global__ void __launch_bounds__(kNormThreads) sens_norm_self_kernel(int64_t n,
 // (no zero guard, src/mlemOperations.hpp:44-54), c += e * a_i.  A row with
 // y_i == 0 is not part of the measurement (the reference's matrix has no row
 // for it) and is skipped.
-template <bool VEC>
 __global__ void __launch_bounds__(kThreads) mlem_project_kernel(int64_t m, const int64_t* __restrict__ rp,
                                                                 const int32_t* __restrict__ col,
                                                                 const float* __restrict__ val,
@@ -308,13 +294,13 @@ __global__ void __launch_bounds__(kThreads) mlem_project_kernel(int64_t m, const
     const float yi = __ldg(y + r);
     if (yi == 0.f) continue;
     const int64_t b = rp[r], e = rp[r + 1];
-    const float yt = row_dot<VEC>(col, val, b, e, x, lane);
+    const float yt = row_dot_seq<8>(col, val, b, e, x, lane);
     const float f = __fdiv_rn(yi, yt);
     if (ll && lane == 0) {
       ly += double(yi) * log(double(yt));
       lt += double(yt);
     }
-    row_scatter<VEC>(col, val, b, e, f, c, lane);
+    row_scatter<8>(col, val, b, e, f, c, lane);
   }
   if (ll) {
     block_add_double(ly, ll);
@@ -554,7 +540,7 @@ __global__ void __launch_bounds__(kThreads, kBackBlocks) mlem_back_kernel(int64_
                                                              double* __restrict__ acc, unsigned long long* next) {
   const int lane = threadIdx.x & 31;
   const double sum = back_columns<UPDATE>(
-      n, cp, x, sens, out, next, [&](int64_t b, int64_t b1) { return row_dot<VEC>(trow, tval, b, b1, e, lane); },
+      n, cp, x, sens, out, next, [&](int64_t b, int64_t b1) { return col_dot<VEC>(trow, tval, b, b1, e, lane); },
       [&](const int64_t(&b)[4], const int(&len)[4]) {
         return short_columns(trow, tval, b, len, e, lane, [](float v) { return v; });
       });
@@ -595,14 +581,8 @@ cudaError_t launch_spmv(int op, int64_t m, int64_t n, const int64_t* rp, const i
       note_launches(1);
     }
     if (m > 0) {
-      if (aligned16(col, val)) {
-        spmv_t_kernel<true><<<row_grid(m), kThreads, 0, s>>>(m, rp, col, val, alpha, x, y);
-        note_launches(1);
-      }
-      else {
-        spmv_t_kernel<false><<<row_grid(m), kThreads, 0, s>>>(m, rp, col, val, alpha, x, y);
-        note_launches(1);
-      }
+      spmv_t_kernel<<<row_grid(m), kThreads, 0, s>>>(m, rp, col, val, alpha, x, y);
+      note_launches(1);
     }
   }
   return cudaGetLastError();
@@ -681,14 +661,8 @@ cudaError_t launch_sens_normalise_self(int64_t n, const double* s64, float* s32,
 cudaError_t launch_mlem_project(int64_t m, const int64_t* rp, const int32_t* col, const float* val, const float* y,
                                 const float* x, float* c, double* d_ll, cudaStream_t s) {
   if (m > 0) {
-    if (aligned16(col, val)) {
-      mlem_project_kernel<true><<<row_grid(m), kThreads, 0, s>>>(m, rp, col, val, y, x, c, d_ll);
-      note_launches(1);
-    }
-    else {
-      mlem_project_kernel<false><<<row_grid(m), kThreads, 0, s>>>(m, rp, col, val, y, x, c, d_ll);
-      note_launches(1);
-    }
+    mlem_project_kernel<<<row_grid(m), kThreads, 0, s>>>(m, rp, col, val, y, x, c, d_ll);
+    note_launches(1);
   }
   return cudaGetLastError();
 }
