@@ -165,7 +165,7 @@ __device__ __forceinline__ void row_scatter(const int32_t* __restrict__ col, con
   }
 }
 
-__global__ void __launch_bounds__(kThreads) spmv_n_kernel(int64_t m, const int64_t* __restrict__ rp,
+__global__ void __launch_bounds__(kThreads, kPassBlocks) spmv_n_kernel(int64_t m, const int64_t* __restrict__ rp,
                                                           const int32_t* __restrict__ col,
                                                           const float* __restrict__ val, float alpha,
                                                           const float* __restrict__ x, float beta,
@@ -559,12 +559,16 @@ unsigned ew_grid(int64_t n) {
   return unsigned(b);
 }
 
-unsigned row_grid(int64_t m) {
+unsigned row_grid(int64_t m, int64_t per_sm = 16) {
   int64_t b = (m * 32 + kThreads - 1) / kThreads;
   if (b < 1) b = 1;
-  if (b > 148 * 16) b = 148 * 16;
+  if (b > 148 * per_sm) b = 148 * per_sm;
   return unsigned(b);
 }
+// Blocks per SM of the SpMV and the row form's projection: the block scheduler
+// evens out the rows better than a longer grid stride (200,000 rows of 724
+// entries: 192 us with 16, 184 with 64; the projection 3 %).
+constexpr int kSpmvGrid = 64;
 
 }  // namespace
 
@@ -572,7 +576,7 @@ cudaError_t launch_spmv(int op, int64_t m, int64_t n, const int64_t* rp, const i
                         float alpha, const float* x, float beta, float* y, cudaStream_t s) {
   if (op == RAPTR_OP_N) {
     if (m > 0) {
-      spmv_n_kernel<<<row_grid(m), kThreads, 0, s>>>(m, rp, col, val, alpha, x, beta, y);
+      spmv_n_kernel<<<row_grid(m, kSpmvGrid), kThreads, 0, s>>>(m, rp, col, val, alpha, x, beta, y);
       note_launches(1);
     }
   } else {
@@ -581,7 +585,7 @@ cudaError_t launch_spmv(int op, int64_t m, int64_t n, const int64_t* rp, const i
       note_launches(1);
     }
     if (m > 0) {
-      spmv_t_kernel<<<row_grid(m), kThreads, 0, s>>>(m, rp, col, val, alpha, x, y);
+      spmv_t_kernel<<<row_grid(m, kSpmvGrid), kThreads, 0, s>>>(m, rp, col, val, alpha, x, y);
       note_launches(1);
     }
   }
@@ -661,7 +665,7 @@ cudaError_t launch_sens_normalise_self(int64_t n, const double* s64, float* s32,
 cudaError_t launch_mlem_project(int64_t m, const int64_t* rp, const int32_t* col, const float* val, const float* y,
                                 const float* x, float* c, double* d_ll, cudaStream_t s) {
   if (m > 0) {
-    mlem_project_kernel<<<row_grid(m), kThreads, 0, s>>>(m, rp, col, val, y, x, c, d_ll);
+    mlem_project_kernel<<<row_grid(m, kSpmvGrid), kThreads, 0, s>>>(m, rp, col, val, y, x, c, d_ll);
     note_launches(1);
   }
   return cudaGetLastError();
