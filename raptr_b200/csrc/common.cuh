@@ -148,41 +148,82 @@ __device__ __forceinline__ bool candidate_test(const DGeom& g, const Channel& ch
   return dist < ch.radius;
 }
 
-// Conservative z-interval of the voxel row (ix, iy) that can pass the
-// cylinder test.  Only prunes the scan: every voxel inside is still decided
-// by candidate_test, and the interval is widened (radius +2%, two voxels on
-// each side) so that it contains every passing voxel.
-__device__ inline bool row_z_interval(const DGeom& g, const Channel& ch, int ix, int iy, int* z0, int* z1) {
-  float inv = 1.0f / ch.abs_ab;
-  float ux = ch.ab[0] * inv, uy = ch.ab[1] * inv, uz = ch.ab[2] * inv;
-  float R = ch.radius * 1.02f + 0.05f * fmaxf(g.d[0], fmaxf(g.d[1], g.d[2]));
-  float dx = g.o[0] + (ix + 0.5f) * g.d[0] - ch.c0[0];
-  float dy = g.o[1] + (iy + 0.5f) * g.d[1] - ch.c0[1];
-  float w = dx * ux + dy * uy;
-  float a2 = 1.0f - uz * uz;
-  float c0 = dx * dx + dy * dy - w * w - R * R;
-  int nz = g.n[2];
-  if (a2 < 1e-6f) {
-    if (c0 < 0.f) { *z0 = 0; *z1 = nz - 1; return true; }
-    return false;
+// The voxel rows (ix, iy, all z) of a channel's enclosing cylinder, from its
+// centre line (unit direction u through c0) and squared radius.  A voxel whose
+// squared distance from the line, in ordinary float arithmetic, is within
+// `margin` of the radius's is decided by candidate_test; the others are settled
+// by their row's intervals.  margin: 2e-3 of r2 (candidate_test itself rounds to
+// 1e-5 of it) and 30 roundings of the squares that cancel in the distance.
+struct CylinderRows {
+  float ux, uy, uz, a2;  // a2 = ux^2 + uy^2
+  float r2;
+};
+
+__device__ __forceinline__ CylinderRows cylinder_rows(const Channel& ch) {
+  CylinderRows c;
+  const float inv = 1.0f / ch.abs_ab;
+  c.ux = ch.ab[0] * inv;
+  c.uy = ch.ab[1] * inv;
+  c.uz = ch.ab[2] * inv;
+  c.a2 = c.ux * c.ux + c.uy * c.uy;
+  c.r2 = ch.radius * ch.radius;
+  return c;
+}
+
+// The rows [*y0, *y1] of slab ix that can hold candidates: a z with distance
+// below R exists where |dy*ux - dx*uy| <= R*sqrt(a2).  One row of margin on
+// each side.
+__device__ __forceinline__ bool slab_rows(const DGeom& g, const Channel& ch, const CylinderRows& c, int ix, int* y0,
+                                          int* y1) {
+  *y0 = 0;
+  *y1 = g.n[1] - 1;
+  if (fabsf(c.ux) < 1e-3f) return true;
+  const float dx = g.o[0] + (ix + 0.5f) * g.d[0] - ch.c0[0];
+  const float mid = dx * c.uy / c.ux, half = 1.01f * ch.radius * sqrtf(c.a2) / fabsf(c.ux);
+  const float lo = (mid - half + ch.c0[1] - g.o[1]) / g.d[1] - 0.5f, hi = (mid + half + ch.c0[1] - g.o[1]) / g.d[1] - 0.5f;
+  const float e = 1.0f + 1e-5f * fabsf(mid) / g.d[1];
+  *y0 = max(0, int(ceilf(fmaxf(lo - e, -1.0f))));
+  *y1 = min(g.n[1] - 1, int(floorf(fminf(hi + e, float(g.n[1])))));
+  return *y0 <= *y1;
+}
+
+// Row (ix, iy): its candidates lie in [*lo, *hi], and all voxels of [*in0, *in1]
+// (empty where in0 > in1) are candidates.
+__device__ __forceinline__ bool row_cells(const DGeom& g, const Channel& ch, const CylinderRows& c, int ix, int iy,
+                                          int* lo, int* hi, int* in0, int* in1) {
+  const int nz = g.n[2];
+  const float dx = g.o[0] + (ix + 0.5f) * g.d[0] - ch.c0[0];
+  const float dy = g.o[1] + (iy + 0.5f) * g.d[1] - ch.c0[1];
+  const float q = dx * dx + dy * dy, w = dx * c.ux + dy * c.uy;
+  const float margin = 2e-3f * c.r2 + 4e-6f * (q + w * w);
+  const float rest = q - w * w;  // squared distance = rest + a2*dz^2 - 2*w*uz*dz
+  *in0 = 0;
+  *in1 = -1;
+  if (c.a2 < 1e-6f) {  // along z
+    *lo = 0;
+    *hi = nz - 1;
+    return true;
   }
-  float b1 = -2.0f * uz * w;
-  float disc = b1 * b1 - 4.0f * a2 * c0;
-  if (disc < 0.f) return false;
-  float sq = sqrtf(disc);
-  float zlo = ch.c0[2] + (-b1 - sq) / (2.f * a2);
-  float zhi = ch.c0[2] + (-b1 + sq) / (2.f * a2);
-  float flo = (zlo - g.o[2]) / g.d[2] - 0.5f;
-  float fhi = (zhi - g.o[2]) / g.d[2] - 0.5f;
-  if (fhi < -3.0f || flo > float(nz) + 2.0f) return false;
-  int lo = int(floorf(flo)) - 2;
-  int hi = int(ceilf(fhi)) + 2;
-  lo = lo < 0 ? 0 : lo;
-  hi = hi > nz - 1 ? nz - 1 : hi;
-  if (lo > hi) return false;
-  *z0 = lo;
-  *z1 = hi;
-  return true;
+  const float B = w * c.uz, inv = 1.0f / c.a2;
+  const float outer = B * B - c.a2 * (rest - c.r2 - margin);
+  if (outer < 0.f) return false;
+  // z index of a distance dz from the crystal centre's z
+  const float at = (ch.c0[2] - g.o[2]) / g.d[2] - 0.5f, scale = inv / g.d[2];
+  const float so = sqrtf(outer), tol = 0.02f + 1e-5f * (fabsf(at) + (fabsf(B) + so) * scale);
+  const float flo = fmaxf(at + (B - so) * scale - tol, -1.0f), fhi = fminf(at + (B + so) * scale + tol, float(nz));
+  if (!(flo <= fhi)) return false;
+  *lo = max(0, int(ceilf(flo)));
+  *hi = min(nz - 1, int(floorf(fhi)));
+  const float inner = B * B - c.a2 * (rest - c.r2 + margin);
+  if (inner > 0.f) {
+    const float si = sqrtf(inner);
+    const float a = fmaxf(at + (B - si) * scale + tol, 0.0f), b = fminf(at + (B + si) * scale - tol, float(nz - 1));
+    if (a <= b) {
+      *in0 = int(ceilf(a));
+      *in1 = int(floorf(b));
+    }
+  }
+  return *lo <= *hi;
 }
 
 // ---------------------------------------------------------------------------
