@@ -210,7 +210,10 @@ struct BatchArgs {
   const int32_t* trow = nullptr;
   const void* tval = nullptr;
   const int32_t* rank = nullptr;
-  const int32_t* col_order = nullptr;  // back-pass column order (may be null)
+  // the columns with entries in the order of the back pass, then the others, and
+  // how many have entries (launch_batch_columns)
+  const int32_t* cols = nullptr;
+  const int64_t* n_full = nullptr;
   const float* Y = nullptr;
   const float* S = nullptr;
   float* X = nullptr;
@@ -230,6 +233,10 @@ struct BatchArgs {
 // seg[j*(B+1) + b] = offset in column j of its first entry with row >= b*m/B.
 cudaError_t launch_block_seg(int64_t n, int64_t m, int B, const int64_t* cp, const int32_t* trow, int32_t* seg,
                              cudaStream_t s);
+// cols (n) of BatchArgs from the column pointers and an order of the columns (null:
+// as they are); flag n, pos n + 1 (pos + n is n_full), scan_tmp scan_temp_elems(n).
+cudaError_t launch_batch_columns(int64_t n, const int64_t* cp, const int32_t* order, int64_t* flag, int64_t* pos,
+                                 int64_t* scan_tmp, int32_t* cols, cudaStream_t s);
 // K frames (a multiple of 4) in tiles of at most kt (4, 8, 16, 32 or 64).
 bool batch_tile_supported(int K, int kt);
 // The tile that starts at frame f0: kt while kt frames remain, else the

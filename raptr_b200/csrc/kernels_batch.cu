@@ -44,10 +44,12 @@ unsigned grid_warps(int64_t items) {
 }
 
 constexpr int kColsPerWarp = 48;  // back pass: columns a warp takes before its block ends
-// CTAs per SM both passes are compiled for: with 5 (48 registers) the back
-// pass runs 10-35 % faster for every frame tile than compiled without a
-// bound (40 registers, 6 CTAs per SM), the forward pass 1-6 % (8: slower)
-constexpr int kBatchBlocks = 5;
+// CTAs per SM the passes are compiled for: 5 forward (48 registers), 4 back (57,122
+// rows of 70^3, 64 frames in tiles of 64 / 16 / 4, back pass with 3, 4, 5, 6: 767,
+// 802, 1059, 827 / 1008, 1037, 1249, 1897 / 1686, 1582, 2139, 2589 us; forward with
+// 3, 4, 5: 643, 601, 606 / 980, 879, 922 / 2005, 1763, 1672, and 5 is 2-4 % faster
+// on 5.14M rows).
+constexpr int kForwardBlocks = 5, kBackBlocks = 4;
 constexpr double kBackGroupBytes = 48.0 * (1 << 20);  // ratios of a back-pass row-block group
 
 __device__ __forceinline__ float to_f(float v) { return v; }
@@ -70,6 +72,34 @@ __device__ __forceinline__ void fma4(float (&a)[4], float w, float4 x) {
   a[3] += w * x.w;
 }
 
+// acc += the entries [b, e) of a row or column times the frames at `at` + index *
+// stride: the lane's slot's entries, its four frames, two entries per slot in
+// flight.  A 64-frame tile has two slots, which keep sums of their own for the two
+// (as many roundings in a row as at 32 frames, four slots).  (Reading 32 entries'
+// indices and values at once and handing them to the slots by shuffles is 10-40 %
+// slower: the slots' loads are broadcasts, and the gathers wait for the shuffles.)
+template <int KT, typename VT>
+__device__ __forceinline__ void gather_entries(const int32_t* __restrict__ idx, const VT* __restrict__ val, int64_t b,
+                                               int64_t e, const float* __restrict__ at, int64_t stride, int lane,
+                                               float (&acc)[4]) {
+  using S = Split<KT>;
+  int64_t k = b + lane / S::LPE;
+  float odd[4] = {0.f, 0.f, 0.f, 0.f};
+  for (; k + S::EPW < e; k += 2 * S::EPW) {
+    const int c0 = __ldg(idx + k), c1 = __ldg(idx + k + S::EPW);
+    const float w0 = to_f(val[k]), w1 = to_f(val[k + S::EPW]);
+    const float4 x0 = ld4(at + int64_t(c0) * stride);
+    const float4 x1 = ld4(at + int64_t(c1) * stride);
+    fma4(acc, w0, x0);
+    fma4(S::EPW > 2 ? acc : odd, w1, x1);
+  }
+  if (k < e) fma4(acc, to_f(val[k]), ld4(at + int64_t(__ldg(idx + k)) * stride));
+  if (S::EPW <= 2) {
+#pragma unroll
+    for (int v = 0; v < 4; v++) acc[v] += odd[v];
+  }
+}
+
 // Forward: Et[rank_i*KT + f - f0] = sc_i * Y[i*K + f] / (sc_i * sum_j v_ij
 // X[j*K + f]) for the frames f of the tile (0 where Y == 0), Et = E + f0*m
 // the tile's block of ratios; sc = rscale (FP16) or 1.  The images are gathered from Xg with row stride xs:
@@ -77,7 +107,7 @@ __device__ __forceinline__ void fma4(float (&a)[4], float w, float4 x) {
 // tile then gathers from n*16 bytes instead of 16 bytes of each 256-byte
 // row of a 64-frame X).
 template <int KT, typename VT>
-__global__ void __launch_bounds__(kThreads, kBatchBlocks) batch_forward_kernel(int64_t m, int K, int f0,
+__global__ void __launch_bounds__(kThreads, kForwardBlocks) batch_forward_kernel(int64_t m, int K, int f0,
                                                                  const int64_t* __restrict__ rp,
                                                                  const int32_t* __restrict__ col,
                                                                  const VT* __restrict__ val,
@@ -96,18 +126,7 @@ __global__ void __launch_bounds__(kThreads, kBatchBlocks) batch_forward_kernel(i
     float acc[S::VEC];
 #pragma unroll
     for (int v = 0; v < S::VEC; v++) acc[v] = 0.f;
-    const int64_t b = rp[r], e = rp[r + 1];
-    int64_t k = b + es;
-    // two entries per slot in flight
-    for (; k + S::EPW < e; k += 2 * S::EPW) {
-      const int c0 = __ldg(col + k), c1 = __ldg(col + k + S::EPW);
-      const float w0 = to_f(val[k]), w1 = to_f(val[k + S::EPW]);
-      const float4 x0 = ld4(X + int64_t(c0) * xs);
-      const float4 x1 = ld4(X + int64_t(c1) * xs);
-      fma4(acc, w0, x0);
-      fma4(acc, w1, x1);
-    }
-    if (k < e) fma4(acc, to_f(val[k]), ld4(X + int64_t(__ldg(col + k)) * xs));
+    gather_entries<KT>(col, val, rp[r], rp[r + 1], X, xs, lane, acc);
 #pragma unroll
     for (int o = S::LPE; o < 32; o <<= 1)
 #pragma unroll
@@ -127,8 +146,9 @@ __global__ void __launch_bounds__(kThreads, kBatchBlocks) batch_forward_kernel(i
 // Back projection and update for the frames of the tile:
 // c = sum_k v_kj Eb[k*KT + f - f0] (Eb = E + f0*m, the tile's block of
 // ratios; FP32, the FP16 values dominate its error),
-// XX = X*c/(S+(S==0)), acc[f] += sum_j XX (FP64).  Warps take columns from
-// the counter *next (zero at launch).
+// XX = X*c/(S+(S==0)), acc[f] += sum_j XX (FP64).  Warps take the columns that
+// have entries (the first *n_full of cols) from the counter *next (zero at
+// launch); the others are batch_empty_kernel's.
 //
 // With a row-block group (seg non-null), only the column's entries whose
 // rows lie in blocks [b0, b1) of the transpose's row order are summed
@@ -138,14 +158,15 @@ __global__ void __launch_bounds__(kThreads, kBatchBlocks) batch_forward_kernel(i
 // last group adds them and finishes as above.  mode: 0 = the whole column
 // at once, 1 = first group, 2 = a middle group, 3 = the last group.
 template <int KT, typename VT>
-__global__ void __launch_bounds__(kThreads, kBatchBlocks) batch_back_kernel(int64_t n, int K, int f0, unsigned long long* next,
+__global__ void __launch_bounds__(kThreads, kBackBlocks) batch_back_kernel(int64_t n, int K, int f0, unsigned long long* next,
                                                               const int64_t* __restrict__ cp,
                                                               const int32_t* __restrict__ trow,
                                                               const VT* __restrict__ tval,
                                                               const float* __restrict__ Eb,
                                                               const float* __restrict__ X,
                                                               const float* __restrict__ sens,
-                                                              const int32_t* __restrict__ col_order,
+                                                              const int32_t* __restrict__ cols,
+                                                              const int64_t* __restrict__ n_full,
                                                               float* __restrict__ XX, double* __restrict__ acc,
                                                               const int32_t* __restrict__ seg, int segw, int b0,
                                                               int b1, int mode, float* __restrict__ P) {
@@ -161,13 +182,14 @@ __global__ void __launch_bounds__(kThreads, kBatchBlocks) batch_back_kernel(int6
   __shared__ double red[KT];  // the block's image sums per frame of the tile
   for (int i = threadIdx.x; i < KT; i += blockDim.x) red[i] = 0.0;
   __syncthreads();
+  const unsigned long long count = (unsigned long long)*n_full;
   for (int taken = 0; taken < kColsPerWarp; taken++) {
     // columns are handed out one at a time (their lengths vary ~20-fold)
     unsigned long long q = 0;
     if (lane == 0) q = atomicAdd(next, 1ull);
     q = __shfl_sync(0xffffffffu, q, 0);
-    if (q >= (unsigned long long)n) break;
-    const int64_t j = col_order ? int64_t(__ldg(col_order + q)) : int64_t(q);
+    if (q >= count) break;
+    const int64_t j = __ldg(cols + q);
     float s[S::VEC];
 #pragma unroll
     for (int v = 0; v < S::VEC; v++) s[v] = 0.f;
@@ -177,16 +199,7 @@ __global__ void __launch_bounds__(kThreads, kBatchBlocks) batch_back_kernel(int6
       b = c0 + __ldg(seg + j * segw + b0);
       e = c0 + __ldg(seg + j * segw + b1);
     }
-    int64_t p = b + es;
-    for (; p + S::EPW < e; p += 2 * S::EPW) {
-      const int k0 = __ldg(trow + p), k1 = __ldg(trow + p + S::EPW);
-      const float w0 = to_f(tval[p]), w1 = to_f(tval[p + S::EPW]);
-      const float4 e0 = ld4(Et + int64_t(k0) * KT);
-      const float4 e1 = ld4(Et + int64_t(k1) * KT);
-      fma4(s, w0, e0);
-      fma4(s, w1, e1);
-    }
-    if (p < e) fma4(s, to_f(tval[p]), ld4(Et + int64_t(__ldg(trow + p)) * KT));
+    gather_entries<KT>(trow, tval, b, e, Et, KT, lane, s);
 #pragma unroll
     for (int o = S::LPE; o < 32; o <<= 1)
 #pragma unroll
@@ -225,6 +238,45 @@ __global__ void __launch_bounds__(kThreads, kBatchBlocks) batch_back_kernel(int6
     if (red[i] != 0.0) atomicAdd(acc + f0 + i, red[i]);
 }
 
+// The update of the columns without entries (cols[*n_full] on, where few views
+// are measured two thirds of them): c = 0, so XX = X*0/(S+(S==0)), which is 0
+// unless X is not finite; acc gets it then.
+__global__ void __launch_bounds__(kThreads) batch_empty_kernel(int64_t n, int K, const int32_t* __restrict__ cols,
+                                                               const int64_t* __restrict__ n_full,
+                                                               const float* __restrict__ X,
+                                                               const float* __restrict__ sens,
+                                                               float* __restrict__ XX, double* __restrict__ acc) {
+  const int64_t first = *n_full;
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < (n - first) * K;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t q = i / K;
+    const int f = int(i - q * K);
+    const int64_t j = __ldg(cols + first + q);
+    float dvs = __ldg(sens + j);
+    dvs += float(dvs == 0.f);
+    const float xx = __fdiv_rn(__fmul_rn(X[j * K + f], 0.f), dvs);
+    XX[j * K + f] = xx;
+    if (xx != 0.f) atomicAdd(acc + f, double(xx));
+  }
+}
+
+// flag[q] = 1 where the q-th column of the order has entries; then, with pos its
+// exclusive sums, cols = those columns in order, followed by the others.
+__global__ void batch_flag_kernel(int64_t n, const int64_t* __restrict__ cp, const int32_t* __restrict__ order,
+                                  int64_t* __restrict__ flag) {
+  const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (q >= n) return;
+  const int64_t j = order ? int64_t(order[q]) : q;
+  flag[q] = cp[j + 1] > cp[j] ? 1 : 0;
+}
+__global__ void batch_columns_kernel(int64_t n, const int64_t* __restrict__ cp, const int32_t* __restrict__ order,
+                                     const int64_t* __restrict__ pos, int32_t* __restrict__ cols) {
+  const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (q >= n) return;
+  const int64_t j = order ? int64_t(order[q]) : q;
+  cols[cp[j + 1] > cp[j] ? pos[q] : pos[n] + q - pos[q]] = int32_t(j);
+}
+
 // Xt[j*t + f'] = X[j*K + f0 + f'], the tile's frames of every image row
 // (t a multiple of 4: one 16-byte copy per thread and step).
 __global__ void batch_tile_images_kernel(int64_t n, int K, int f0, int t, const float* __restrict__ X,
@@ -237,13 +289,20 @@ __global__ void batch_tile_images_kernel(int64_t n, int K, int f0, int t, const 
   }
 }
 
-// X = XX * (1 / acc[f]) for all frames; then acc = 0 for the next pass.
-__global__ void batch_normalise_kernel(int64_t n, int K, float* __restrict__ X, const float* __restrict__ XX,
-                                       const double* __restrict__ acc) {
-  const int64_t total = n * K;
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
-    const int f = int(i % K);
-    X[i] = XX[i] * float(1.0 / acc[f]);
+// X = XX * (1 / acc[f]) for all frames.  A thread's four frames stay the same (the
+// grid's threads are a multiple of K / 4), so their scales are taken once.
+__global__ void batch_normalise_kernel(int64_t n, int K, int64_t threads, float* __restrict__ X,
+                                       const float* __restrict__ XX, const double* __restrict__ acc) {
+  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (t >= threads) return;
+  const int f = int(t % (K / 4)) * 4;
+  float sc[4];
+#pragma unroll
+  for (int v = 0; v < 4; v++) sc[v] = float(1.0 / acc[f + v]);
+  const int64_t total = n * (K / 4);
+  for (int64_t i = t; i < total; i += threads) {
+    const float4 x = reinterpret_cast<const float4*>(XX)[i];
+    reinterpret_cast<float4*>(X)[i] = make_float4(x.x * sc[0], x.y * sc[1], x.z * sc[2], x.w * sc[3]);
   }
 }
 
@@ -269,10 +328,12 @@ cudaError_t launch_tile(const BatchArgs& a, bool forward, int f0, double* acc, u
         a.m, a.K, f0, a.rp, a.col, static_cast<const VT*>(a.val), a.half ? a.rscale : nullptr, a.Y,
         compact ? a.Xt : a.X + f0, compact ? KT : a.K, a.rank, a.E + int64_t(f0) * a.m);
   } else {
-    batch_back_kernel<KT, VT><<<unsigned((a.n + kColsPerWarp * (kThreads / 32) - 1) / (kColsPerWarp * (kThreads / 32))),
-                                kThreads, 0, s>>>(a.n, a.K, f0, next, a.cp, a.trow, static_cast<const VT*>(a.tval),
+    // blocks for kColsPerWarp columns a warp, and enough to fill the GPU
+    const int64_t per = kColsPerWarp * (kThreads / 32);
+    const int64_t blocks = std::min<int64_t>(std::max<int64_t>((a.n + per - 1) / per, 148 * 10), grid_warps(a.n));
+    batch_back_kernel<KT, VT><<<unsigned(blocks), kThreads, 0, s>>>(a.n, a.K, f0, next, a.cp, a.trow, static_cast<const VT*>(a.tval),
                                                   a.E + int64_t(f0) * a.m,
-                                                  a.X, a.S, a.col_order, a.XX, acc, grp.mode ? a.seg : nullptr,
+                                                  a.X, a.S, a.cols, a.n_full, a.XX, acc, grp.mode ? a.seg : nullptr,
                                                   a.seg_blocks + 1, grp.b0, grp.b1, grp.mode, a.P);
   }
   note_launches(1);
@@ -334,6 +395,19 @@ int batch_tile_at(int K, int kt, int f0) {
   return t;
 }
 
+cudaError_t launch_batch_columns(int64_t n, const int64_t* cp, const int32_t* order, int64_t* flag, int64_t* pos,
+                                 int64_t* scan_tmp, int32_t* cols, cudaStream_t s) {
+  const unsigned blocks = unsigned((n + kThreads - 1) / kThreads);
+  batch_flag_kernel<<<blocks, kThreads, 0, s>>>(n, cp, order, flag);
+  note_launches(1);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = launch_scan_i64(flag, n, pos, scan_tmp, s);
+  if (e != cudaSuccess) return e;
+  batch_columns_kernel<<<blocks, kThreads, 0, s>>>(n, cp, order, pos, cols);
+  note_launches(1);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_batch_iteration(const BatchArgs& a, int kt, double* acc, unsigned long long* next, cudaStream_t s,
                                    cudaEvent_t ev_mid) {
   // Tiles of kt frames while that many remain, then the largest power of
@@ -363,10 +437,9 @@ cudaError_t launch_batch_iteration(const BatchArgs& a, int kt, double* acc, unsi
     }
     return out;
   };
-  const int ngroups_max = a.seg_blocks > 0 ? a.seg_blocks : 1;
   cudaError_t e = cudaMemsetAsync(acc, 0, size_t(a.K) * sizeof(double), s);
   if (e == cudaSuccess)
-    e = cudaMemsetAsync(next, 0, size_t(a.K / 4) * size_t(ngroups_max) * sizeof(unsigned long long), s);
+    e = cudaMemsetAsync(next, 0, size_t(a.K / 4) * size_t(std::max(a.seg_blocks, 1)) * sizeof(unsigned long long), s);
   const BackGroup whole;
   for (int f0 = 0; f0 < a.K && e == cudaSuccess; f0 += batch_tile_at(a.K, kt, f0)) {
     const int t = batch_tile_at(a.K, kt, f0);
@@ -374,21 +447,22 @@ cudaError_t launch_batch_iteration(const BatchArgs& a, int kt, double* acc, unsi
                : launch_tile_kt<float>(t, a, true, f0, acc, nullptr, whole, s);
   }
   if (e == cudaSuccess && ev_mid) e = cudaEventRecord(ev_mid, s);
-  int counter = 0;
   for (int f0 = 0; f0 < a.K && e == cudaSuccess; f0 += batch_tile_at(a.K, kt, f0)) {
     const int t = batch_tile_at(a.K, kt, f0);
     for (const BackGroup& q : groups(t)) {
       if (e != cudaSuccess) break;
-      e = a.half ? launch_tile_kt<__half>(t, a, false, f0, acc, next + counter, q, s)
-                 : launch_tile_kt<float>(t, a, false, f0, acc, next + counter, q, s);
-      counter++;
+      e = a.half ? launch_tile_kt<__half>(t, a, false, f0, acc, next, q, s)
+                 : launch_tile_kt<float>(t, a, false, f0, acc, next, q, s);
+      next++;
     }
   }
   if (e == cudaSuccess) {
-    const int64_t total = a.n * a.K;
-    int64_t blocks = (total + kThreads - 1) / kThreads;
-    if (blocks > 148 * 8) blocks = 148 * 8;
-    batch_normalise_kernel<<<unsigned(blocks), kThreads, 0, s>>>(a.n, a.K, a.X, a.XX, acc);
+    batch_empty_kernel<<<148 * 8, kThreads, 0, s>>>(a.n, a.K, a.cols, a.n_full, a.X, a.S, a.XX, acc);
+    note_launches(1);
+    const int64_t q = a.K / 4;
+    const int64_t threads = std::min<int64_t>(a.n * q, std::max<int64_t>(int64_t(148) * 8 * kThreads / q, 1) * q);
+    batch_normalise_kernel<<<unsigned((threads + kThreads - 1) / kThreads), kThreads, 0, s>>>(a.n, a.K, threads, a.X,
+                                                                                             a.XX, acc);
     note_launches(1);
     e = cudaGetLastError();
   }
