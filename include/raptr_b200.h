@@ -241,7 +241,8 @@ raptr_status raptr_sensitivity_csc(int64_t n, const int64_t* d_col_ptr, const fl
                                    float* d_s32, void* stream);
 
 typedef struct raptr_mlem_opts {
-  int32_t use_graph;   /* capture the iteration loop in a CUDA graph            */
+  int32_t use_graph;   /* return when the iterations have ended (they are plain
+                        * launches: a CUDA graph of them is slower at any size) */
   double* h_loglik;    /* optional: per-iteration Poisson log-likelihood (FP64)  */
   float* h_kernel_ms;  /* optional: 2*n_iter device times (ms) of the two passes of
                           each iteration, from CUDA events on the stream; when
@@ -375,7 +376,7 @@ raptr_status raptr_mlem_f64(raptr_ctx* ctx, int64_t m, int64_t n, const int64_t*
  * frame_tile frames while that many remain, then the largest power of two
  * that fits (40 frames at 32: 32 + 8).  d_x and d_y must be 16-byte
  * aligned.
- * opts: use_graph captures the n_iter iterations in a CUDA graph;
+ * opts: with use_graph the call returns when the iterations have ended;
  * h_kernel_ms receives per iteration the forward and back-pass times. */
 raptr_status raptr_mlem_batch(raptr_ctx* ctx, int64_t m, int64_t n, int32_t n_frames, int32_t value_type,
                               const int64_t* d_row_ptr, const int32_t* d_col, const void* d_val,
