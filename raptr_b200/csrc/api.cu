@@ -220,6 +220,20 @@ struct raptr_ctx {
     return cudaSuccess;
   }
 
+  // The streams and events of a pipelined build, made on its first use: making
+  // them anew took 0.2 ms of every build.
+  cudaStream_t placement = nullptr, rows2 = nullptr;
+  cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+
+  cudaError_t build_streams() {
+    cudaError_t e = cudaSuccess;
+    if (!placement) e = cudaStreamCreateWithFlags(&placement, cudaStreamNonBlocking);
+    if (e == cudaSuccess && !rows2) e = cudaStreamCreateWithFlags(&rows2, cudaStreamNonBlocking);
+    for (auto& v : ev)
+      if (e == cudaSuccess && !v) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
+    return e;
+  }
+
   raptr_status ensure_scratch(size_t bytes) {
     if (bytes <= scratch_bytes) return RAPTR_OK;
     if (d_scratch) dev_free(d_scratch);
@@ -287,6 +301,12 @@ struct Carve {
 };
 
 constexpr size_t kStagingBudget = size_t(1) << 30;  // bytes of row staging per chunk
+
+// Rows of a chunk of a build.
+int64_t rows_per_chunk(int level) {
+  const int64_t per = int64_t(kStagingBudget / (size_t(sm_level_capacity(level)) * 8));
+  return std::min<int64_t>(std::max<int64_t>(per, 1), 65536);
+}
 
 // Output of a build: caller buffers (fixed capacity) or a library matrix
 // that grows.
@@ -361,32 +381,14 @@ struct Builder {
   // rebuilt at the next level by rows(), and the pipeline restarts after it.
   raptr_status rows_pipelined(int level, int64_t row0, int64_t nrows) {
     const int H = sm_level_capacity(level);
-    int64_t per = std::max<int64_t>(1, int64_t(kStagingBudget / (size_t(H) * 8)));
-    per = std::min<int64_t>(per, 65536);
+    const int64_t per = rows_per_chunk(level);
     if (!ctx->h_pin) RCU(cudaMallocHost(&ctx->h_pin, 16 * sizeof(int64_t)));
     // words 0-1: the slab kernel's flags, 2-3: the table kernel's (per buffer)
     volatile int32_t* h_flags = reinterpret_cast<volatile int32_t*>(ctx->h_pin);
     volatile int64_t* h_total = ctx->h_pin + 2;
-    cudaStream_t P = nullptr, S2 = nullptr;
-    cudaEvent_t ev_k[2] = {nullptr, nullptr}, ev_g[2] = {nullptr, nullptr}, ev_j = nullptr;
-    auto release = [&]() {
-      for (auto e : ev_k) if (e) cudaEventDestroy(e);
-      for (auto e : ev_g) if (e) cudaEventDestroy(e);
-      if (ev_j) cudaEventDestroy(ev_j);
-      if (P) cudaStreamDestroy(P);
-      if (S2) cudaStreamDestroy(S2);
-    };
-    struct Guard {
-      std::function<void()> f;
-      ~Guard() { f(); }
-    } guard{release};
-    RCU(cudaStreamCreateWithFlags(&P, cudaStreamNonBlocking));
-    RCU(cudaStreamCreateWithFlags(&S2, cudaStreamNonBlocking));
-    for (int b = 0; b < 2; b++) {
-      RCU(cudaEventCreateWithFlags(&ev_k[b], cudaEventDisableTiming));
-      RCU(cudaEventCreateWithFlags(&ev_g[b], cudaEventDisableTiming));
-    }
-    RCU(cudaEventCreateWithFlags(&ev_j, cudaEventDisableTiming));
+    RCU(ctx->build_streams());
+    cudaStream_t P = ctx->placement, S2 = ctx->rows2;
+    cudaEvent_t *ev_k = ctx->ev, *ev_g = ctx->ev + 2, ev_j = ctx->ev[4];
     auto drain = [&]() -> cudaError_t {
       cudaError_t e = cudaStreamSynchronize(s);
       cudaError_t e2 = cudaStreamSynchronize(S2);
@@ -528,12 +530,60 @@ struct Builder {
     return RAPTR_OK;
   }
 
+  // Rows that are one chunk, on the caller's stream with one wait: rows, scan and
+  // gather one after the other (the gather writes within the caller's capacity,
+  // or after the output has grown).  A row that overflows its table is found at
+  // the end, and rows() builds the chunk again a level up.  The pipeline has
+  // nothing to overlap here, and its waits took longer than a few hundred rows
+  // (500 rows of 40^3 x 100 rays: 0.31 ms, so 0.08).
+  raptr_status rows_single(int level) {
+    const int H = sm_level_capacity(level);
+    const int64_t k = n_list;
+    if (!ctx->h_pin) RCU(cudaMallocHost(&ctx->h_pin, 16 * sizeof(int64_t)));
+    RCHECK(ctx->ensure_scratch(Carve::need({size_t(k) * H * sizeof(int32_t), size_t(k) * H * sizeof(float),
+                                            size_t(k) * sizeof(int32_t)})));
+    Carve cv(ctx->d_scratch);
+    int32_t* st_col = cv.take<int32_t>(size_t(k) * H);
+    float* st_val = cv.take<float>(size_t(k) * H);
+    int32_t* row_nnz = cv.take<int32_t>(size_t(k));
+    const double t0 = trace_on() ? trace_ms() : 0.0;
+    // the entry count (cleared by the caller) and, in the next word, the flags
+    int32_t* d_flags = reinterpret_cast<int32_t*>(ctx->d_i64 + 1);
+    volatile int64_t* h = ctx->h_pin;
+    RCU(cudaMemsetAsync(d_flags, 0, sizeof(int64_t), s));
+    RCU(launch_sm_rows(level, ctx->dg, ctx->d_sincos, d_cnl, 0, k, nrays, seed, d_rays, st_col, st_val, row_nnz,
+                       d_flags, s, ctx->d_flags + 4));
+    RCU(launch_rows_scan(row_nnz, k, out.rp, ctx->d_i64, s));
+    if (!out.grow && out.cap > 0)
+      RCU(launch_rows_gather(st_col, st_val, H, out.rp, k, out.cap, out.col, out.val, s));
+    RCU(cudaMemcpyAsync(const_cast<int64_t*>(h), ctx->d_i64, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    RCU(cudaStreamSynchronize(s));
+    const int32_t flags = int32_t(h[1]);
+    if (flags & 4) return fail(RAPTR_ERR_INVALID, "a channel id is outside [0, number of channels)");
+    if (flags & 2) return fail(RAPTR_ERR_OVERFLOW, "ray walk did not terminate (internal error)");
+    if (flags & 1) {
+      if (level + 1 >= sm_num_levels())
+        return fail(RAPTR_ERR_OVERFLOW, "a row has more distinct voxels than the largest per-row table holds");
+      RCU(cudaMemsetAsync(ctx->d_i64, 0, sizeof(int64_t), s));
+      return rows(level + 1, 0, k);
+    }
+    total = h[0];
+    rows_done = k;
+    if (trace_on())
+      trace("build rows 0+%lld level %d: rows and placement %.2f ms, %lld entries", (long long)k, level,
+            trace_ms() - t0, (long long)total);
+    if (out.grow) {
+      RCHECK(ensure_capacity(out, total, rows_done, s));
+      RCU(launch_rows_gather(st_col, st_val, H, out.rp, k, out.cap, out.col, out.val, s));
+    }
+    return RAPTR_OK;
+  }
+
   // Builds rows [row0, row0+nrows) at `level`, retrying at higher levels on
   // table overflow, and places them.
   raptr_status rows(int level, int64_t row0, int64_t nrows) {
     const int H = sm_level_capacity(level);
-    int64_t per = std::max<int64_t>(1, int64_t(kStagingBudget / (size_t(H) * 8)));
-    per = std::min<int64_t>(per, 65536);
+    const int64_t per = rows_per_chunk(level);
     for (int64_t r = row0; r < row0 + nrows; r += per) {
       const int64_t k = std::min(per, row0 + nrows - r);
       size_t need = Carve::need({size_t(k) * H * sizeof(int32_t), size_t(k) * H * sizeof(float),
@@ -605,6 +655,8 @@ raptr_status run_build(raptr_ctx* ctx, const int32_t* d_cnl, int64_t n_list, int
     const int level = sm_pick_level(ctx->dg, nrays);
     if (b.keep_zeros)
       RCHECK(b.rows(level, 0, n_list));
+    else if (n_list <= rows_per_chunk(level))
+      RCHECK(b.rows_single(level));
     else
       RCHECK(b.rows_pipelined(level, 0, n_list));
   }
@@ -678,6 +730,10 @@ raptr_status raptr_ctx_destroy(raptr_ctx* ctx) {
   dev_free(ctx->d_col_order);
   dev_free(ctx->d_bseg);
   cudaFreeHost(ctx->h_pin);
+  if (ctx->placement) cudaStreamDestroy(ctx->placement);
+  if (ctx->rows2) cudaStreamDestroy(ctx->rows2);
+  for (auto v : ctx->ev)
+    if (v) cudaEventDestroy(v);
   delete ctx;
   return RAPTR_OK;
 }
@@ -1827,8 +1883,7 @@ raptr_status raptr_mlem_stream(raptr_ctx* ctx, const int32_t* d_cnl, int64_t n_l
   // the resident CSR.
   auto sweep = [&](bool first, int64_t from) -> raptr_status {
     const int H = sm_level_capacity(level);
-    int64_t per = std::max<int64_t>(1, int64_t(kStagingBudget / (size_t(H) * 8)));
-    per = std::min<int64_t>(per, 65536);
+    int64_t per = rows_per_chunk(level);
     // fewer rows per chunk when the device (or the library's memory limit)
     // has less room than the usual staging
     const size_t room = dev_available(ctx->device) + ctx->scratch_bytes;

@@ -562,7 +562,6 @@ struct alignas(16) SlabRay {
 static_assert(sizeof(SlabRay) == 112, "seven 16-byte loads");
 
 constexpr int kSlabs = 3;               // neighbouring slabs a thread owns (odd: an even number of planes)
-constexpr int kSlabBatch = 192;              // rays staged in shared memory at a time
 constexpr float kIndexMagic = 12582912.f;  // 1.5 * 2^23: adding it rounds to an integer held in the low mantissa bits
 constexpr unsigned kIndexBits = 0x4B400000u;
 
@@ -780,6 +779,7 @@ struct SlabShape {
   int threads = 0;
   int acc_floats = 0;
   int stage_floats = 0;
+  int batch = 0;  // rays staged at a time
   size_t smem() const { return size_t(acc_floats + stage_floats) * 4; }
 };
 
@@ -799,7 +799,8 @@ struct SlabShape {
 // decodes outside the grid is noticed: both send the row to the table.
 __global__ void __launch_bounds__(kSlabThreads, kSlabBlocks)
     sm_slab_kernel(DGeom g, const float2* __restrict__ sincos, const int32_t* __restrict__ cnl_ids, int64_t row0,
-                   int nrays, uint32_t seed, int H, int acc_floats, int stage_floats, int32_t* __restrict__ st_col,
+                   int nrays, uint32_t seed, int H, int acc_floats, int stage_floats, int batch,
+                   int32_t* __restrict__ st_col,
                    float* __restrict__ st_val, int32_t* __restrict__ row_nnz, int32_t* __restrict__ flags,
                    int32_t* __restrict__ reasons) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -828,32 +829,56 @@ __global__ void __launch_bounds__(kSlabThreads, kSlabBlocks)
       if (reasons) atomicAdd(reasons + why, 1);
     }
   };
-  if (tid == 0) {
-    channel_setup(g, sincos, cnl, ch);
-    bad_walk = 0;
-    to_table = 0;
-    outside = 0;
-    win_u = 0;
-    win_v = 0;
-    zbox[0] = zbox[2] = INT_MAX;
-    zbox[1] = zbox[3] = INT_MIN;
-  } else if (tid >= 32) {
+  if (warp == 0) {
+    // The crystals are boxes rotated about y: four corners in (x, z), two bounds
+    // in y.  Lanes 0-3 take the first crystal's corners, 4-7 the second's, each
+    // with the crystal's transform (channel_setup does the same one after the
+    // other in one thread).
+    const ChannelIds id = channel_split(g, cnl);
+    const float2 sc = sincos[id.ida];
+    const int b = (lane >> 2) & 1, c = lane & 3;
+    float m[12], p[3], mid[3];
+    trafo_matrix(m, b == 0 ? g.pos0x : g.pos1x, b == 0 ? id.id0z : id.id1z, b == 0 ? id.id0y : id.id1y,
+                 b == 0 ? g.n0y : g.n1y, b == 0 ? g.n0z : g.n1z, g.segx, g.segy, g.segz, sc.x, sc.y);
+    trafo_apply(m, float(c & 1), float(c >> 1), float(c >> 1), p);
+    trafo_apply(m, 0.5f, 0.5f, 0.5f, mid);
+    if (lane < 8) {
+      corner_x[b][c] = p[0];
+      corner_z[b][c] = p[2];
+      if ((c & 1) == 0) corner_y[b][c >> 1] = p[1];
+    }
+    if (lane < 8 && c == 0) {
+      float* to = b == 0 ? ch.m0 : ch.m1;
+#pragma unroll
+      for (int k = 0; k < 12; k++) to[k] = m[k];
+    }
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const float other = __shfl_sync(0xffffffffu, mid[d], 4);
+      if (lane == 0) {
+        ch.c0[d] = mid[d];
+        ch.ab[d] = RFSUB(other, mid[d]);
+      }
+    }
+    if (lane == 0) {
+      bad_walk = 0;
+      to_table = 0;
+      outside = 0;
+      win_u = 0;
+      win_v = 0;
+      zbox[0] = zbox[2] = INT_MAX;
+      zbox[1] = zbox[3] = INT_MIN;
+    }
+  } else {
     // the other warps clear the sums meanwhile
     float4* a4 = reinterpret_cast<float4*>(acc);
     for (int i = tid - 32; i < acc_floats / 4; i += T - 32) a4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __syncthreads();
-  if (tid < 8) {
-    // the crystals are boxes rotated about y: four corners in (x, z), two
-    // bounds in y
-    const int b = tid >> 2, c = tid & 3;
-    float p[3];
-    trafo_apply(b == 0 ? ch.m0 : ch.m1, float(c & 1), float(c >> 1), float(c >> 1), p);
-    corner_x[b][c] = p[0];
-    corner_z[b][c] = p[2];
-    if ((c & 1) == 0) corner_y[b][c >> 1] = p[1];
+  if (tid == T - 1) {  // what the cylinder test needs, for later
+    ch.abs_ab = norm3_exact(ch.ab[0], ch.ab[1], ch.ab[2]);
+    ch.radius = RFMUL(0.5f, RFADD(norm3_exact(g.d[0], g.d[1], g.d[2]), norm3_exact(g.segx, g.segy, g.segz)));
   }
-  __syncthreads();
   // the slab axis: of x and z, the one along which the crystals lie on
   // opposite sides of the grid, the channel's dominant direction first
   int A = -1, sdir = 0;
@@ -935,7 +960,7 @@ __global__ void __launch_bounds__(kSlabThreads, kSlabBlocks)
   const int wu = win_u, wv = max(win_v, 2), W = wu * wv;
   const int nt = (na + kSlabs - 1) / kSlabs;  // threads of a group
   int G = T / nt;
-  G = min(G, kSlabBatch);
+  G = min(G, batch);
   while (G > 0 && (long long)(kSlabs * W + 3) * ((G * nt + 31) & ~31) > (long long)acc_floats) G--;
   const int Wp = W | 1;  // odd: slots of neighbouring slabs fall into different banks
   if (G == 0 || (long long)na * Wp > (long long)stage_floats) {
@@ -966,7 +991,7 @@ __global__ void __launch_bounds__(kSlabThreads, kSlabBlocks)
   }
   const unsigned spare = unsigned((kSlabs * W * S + (works ? tid : 0)) * 4);
   const f32x2 o2 = pack2(axis_o(g, iu_ax), axis_o(g, iv_ax));
-  const int per = kSlabBatch / G * G;  // as many rays for every group
+  const int per = batch / G * G;  // as many rays for every group
   for (int base = 0; base < nrays; base += per) {
     const int cnt = min(per, nrays - base);
     __syncthreads();  // the batch before is done with
@@ -1301,12 +1326,16 @@ constexpr int kNumLevels = 4;
 // groups.  60,000 rows of 70^3 x 1000 rays / 12,345 of 100^3 x 999: 13.45 /
 // 4.76 ms; with 96 threads 13.9 / 6.4, 256: 15.1 / 4.8, 288: 15.2 / 5.9; with
 // room for four blocks (W = 16-18) 14.5-16.4 / 6.2-6.9, with two slabs per
-// thread 15.0 / 4.8, with one 17.3 / 5.9.
-SlabShape slab_shape(const DGeom& g) {
+// thread 15.0 / 4.8, with one 17.3 / 5.9.  With few rays a row's set-up and
+// compaction are most of it, and more, smaller blocks overlap them: 142,805 rows
+// of 40^3 x 100 rays 5.0 ms with 192 threads, 4.55 with 128 (at 300 rays 1.90 and
+// 1.82 ms for 30,000 rows, at 1000 rays even or slower).
+SlabShape slab_shape(const DGeom& g, int nrays) {
   SlabShape sh;
+  const int most = nrays <= 256 ? 128 : kSlabThreads;
   // the most threads whose groups leave few of them idle
   double best = 0.0;
-  for (int T = kSlabThreads; T >= 128; T -= 32) {
+  for (int T = most; T >= 128; T -= 32) {
     double used = 0.0;
     for (int a = 0; a < 3; a += 2) {
       const int nt = (g.n[a] + kSlabs - 1) / kSlabs;
@@ -1320,7 +1349,8 @@ SlabShape slab_shape(const DGeom& g) {
   const double wy = g.segy / g.d[1] + 2.1, wh = 1.5 * g.segz / std::min(g.d[0], g.d[2]) + 2.1;
   const int W = int(std::min(std::ceil(wy * wh), 64.0));
   sh.acc_floats = (kSlabs * W + 3) * sh.threads;
-  sh.stage_floats = std::max(kSlabBatch * int(sizeof(SlabRay) / 4), std::min(50 * std::max(g.n[0], g.n[2]), 8192));
+  sh.batch = most;
+  sh.stage_floats = std::max(sh.batch * int(sizeof(SlabRay) / 4), std::min(50 * std::max(g.n[0], g.n[2]), 8192));
   return sh;
 }
 
@@ -1343,12 +1373,12 @@ cudaError_t launch_level(const DGeom& g, const float2* d_sincos, const int32_t* 
     return cudaGetLastError();
   }
   if (parts & 1) {
-    const SlabShape sh = slab_shape(g);
+    const SlabShape sh = slab_shape(g, nrays);
     e = cudaFuncSetAttribute(sm_slab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sh.smem()));
     if (e != cudaSuccess) return e;
     sm_slab_kernel<<<unsigned(nrows), unsigned(sh.threads), sh.smem(), s>>>(
-        g, d_sincos, d_cnl, row0, nrays, seed, H, sh.acc_floats, sh.stage_floats, st_col, st_val, row_nnz, d_flags,
-        d_reasons);
+        g, d_sincos, d_cnl, row0, nrays, seed, H, sh.acc_floats, sh.stage_floats, sh.batch, st_col, st_val, row_nnz,
+        d_flags, d_reasons);
     note_launches(1);
   }
   if (parts & 2) {
@@ -1375,10 +1405,17 @@ __global__ void __launch_bounds__(1024) rows_scan_kernel(const TCount* __restric
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) carry = *d_base;
   __syncthreads();
-  for (int64_t t0 = 0; t0 < n; t0 += 1024) {
-    int64_t i = t0 + tid;
-    long long v = (i < n) ? (long long)row_nnz[i] : 0;
-    v = v < 0 ? 0 : v;
+  constexpr int U = 8;  // rows of a thread
+  for (int64_t t0 = 0; t0 < n; t0 += 1024 * U) {
+    const int64_t i = t0 + int64_t(tid) * U;
+    long long c[U];
+    long long v = 0;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      c[u] = i + u < n ? (long long)row_nnz[i + u] : 0;
+      c[u] = c[u] < 0 ? 0 : c[u];
+      v += c[u];
+    }
     long long x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -1398,7 +1435,11 @@ __global__ void __launch_bounds__(1024) rows_scan_kernel(const TCount* __restric
     }
     __syncthreads();
     long long excl = carry + (warp > 0 ? warp_sums[warp - 1] : 0) + x - v;
-    if (i < n) row_ptr[i] = excl;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (i + u < n) row_ptr[i + u] = excl;
+      excl += c[u];
+    }
     __syncthreads();
     if (tid == 0) carry += warp_sums[31];
     __syncthreads();
