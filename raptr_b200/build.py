@@ -27,6 +27,7 @@ UNITS = {
     "kernels_util.cu": [],
     "kernels_mlem.cu": [],
     "kernels_transpose.cu": [],
+    "kernels_transpose_sorted.cu": [],
     "kernels_precision.cu": [],
     "kernels_batch.cu": [],
     "server.cu": [],

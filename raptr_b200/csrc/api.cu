@@ -937,7 +937,68 @@ raptr_status transpose_impl(int64_t m, int64_t n, const int64_t* d_row_ptr, cons
   RCU(cudaMemcpyAsync(&nnz, d_row_ptr + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   RCU(cudaStreamSynchronize(s));
   if (nnz > 0 && (!d_col || !d_val || !d_row_idx || !d_tval)) return fail(RAPTR_ERR_INVALID, "null buffer");
-  // radix sort by column when it applies and its staging (12 bytes per
+  // Rows with ascending columns (every matrix the library builds) are partitioned
+  // without ranking; the kernels notice other rows, before the staging (10 bytes
+  // per entry) is allocated.
+  SortedPlan sorted;
+  if (transpose_sorted_plan(m, n, nnz, &sorted)) {
+    SortedScratch w;
+    const double t0 = trace_on() ? trace_ms() : 0.0;
+    const int64_t tasks = int64_t(sorted.bins) * sorted.blocks, nh = sorted_hist_elems(sorted);
+    // each call's buffers are one allocation, laid out twice: for its size, then for the pointers
+    char *base = nullptr, *small = nullptr, *staging = nullptr;
+    size_t bytes = 0;
+    auto part = [&](auto*& ptr, int64_t count) {
+      if (base) ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(base + bytes);
+      bytes += (size_t(count) * sizeof(*ptr) + 255) & ~size_t(255);
+    };
+    auto lay_small = [&](char* p) {
+      base = p;
+      bytes = 0;
+      part(w.begin, m);
+      part(w.size, tasks);
+      part(w.off, tasks + 1);
+      part(w.scan_tmp, scan_temp_elems(std::max(nh, tasks)));
+      part(w.tile_first, sorted.bins + 1);
+      part(w.flags, 1);
+      part(w.split, int64_t(sorted.bins + 1) * m);
+    };
+    auto lay_staging = [&](char* p) {
+      base = p;
+      bytes = 0;
+      part(w.hist, nh);
+      part(w.place, nh + 1);
+      part(w.st_k, nnz);
+      part(w.st_v, nnz);
+      part(w.st_low, nnz);
+    };
+    int32_t h_flags = -1;  // the ways below may need less memory
+    cudaError_t e = cudaSuccess;
+    lay_small(nullptr);
+    if (dev_malloc(&small, bytes) == cudaSuccess) {
+      lay_small(small);
+      e = launch_sorted_split(sorted, m, n, nnz, d_row_ptr, d_col, d_order, w, s);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(&h_flags, w.flags, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
+      const cudaError_t e2 = cudaStreamSynchronize(s);
+      if (e == cudaSuccess) e = e2;
+      lay_staging(nullptr);
+      if (e == cudaSuccess && h_flags == 0 && dev_malloc(&staging, bytes) == cudaSuccess) {
+        lay_staging(staging);
+        e = launch_sorted_move(sorted, m, n, nnz, d_col, d_val, w, d_col_ptr, d_row_idx, d_tval, s);
+        const cudaError_t e3 = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) e = e3;
+      }
+    }
+    const bool done = staging != nullptr;
+    if (e == cudaSuccess && !done) (void)cudaGetLastError();
+    dev_free(staging);
+    dev_free(small);
+    if (trace_on()) trace("transpose of sorted rows: %.2f ms, flags %d", trace_ms() - t0, int(h_flags));
+    if (e != cudaSuccess) return cuda_fail(e, "raptr_csr_transpose");
+    if (h_flags > 0 && (h_flags & 1)) return fail(RAPTR_ERR_INVALID, "column index or row order entry out of range");
+    if (done) return RAPTR_OK;
+  }
+  // Otherwise: radix sort by column when it applies and its staging (12 bytes per
   // entry) fits; else the blocked transpose (4 bytes per column and block)
   RadixPlan plan;
   if (nnz > 0 && transpose_radix_plan(m, n, nnz, &plan)) {

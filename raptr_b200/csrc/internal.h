@@ -278,6 +278,40 @@ cudaError_t launch_transpose_radix(const RadixPlan& p, int64_t m, int64_t n, int
                                    int32_t* st_key, int32_t* st_k, float* st_v, int32_t* bad, int64_t* cp,
                                    int32_t* trow, float* tval, cudaStream_t s);
 
+// CSR -> CSC of rows with strictly ascending columns (kernels_transpose_sorted.cu),
+// in two calls.  The first finds the pieces and sets *flags: 0 = go on; 1 = a column
+// or order entry out of range; 2 = columns that do not ascend, or a row of more
+// than 65535; 4 = the rows taken do not hold nnz entries.  The second moves the
+// entries, and does nothing unless *flags is 0.
+struct SortedPlan {
+  int bins = 0, rows_per_block = 0, blocks = 0;
+  int64_t max_tiles = 0;
+};
+struct SortedScratch {
+  // both calls
+  int64_t* begin = nullptr;       // m
+  int64_t* off = nullptr;         // bins * blocks + 1
+  int64_t* scan_tmp = nullptr;    // scan_temp_elems of bins * blocks or sorted_hist_elems, the larger
+  int32_t* tile_first = nullptr;  // bins + 1
+  int32_t* flags = nullptr;       // 1
+  uint16_t* split = nullptr;      // (bins + 1) * m
+  // the first
+  int64_t* size = nullptr;        // bins * blocks
+  // the second
+  int64_t* hist = nullptr;        // sorted_hist_elems
+  int64_t* place = nullptr;       // sorted_hist_elems + 1
+  int32_t* st_k = nullptr;        // nnz each
+  float* st_v = nullptr;
+  uint16_t* st_low = nullptr;
+};
+bool transpose_sorted_plan(int64_t m, int64_t n, int64_t nnz, SortedPlan* p);
+int64_t sorted_hist_elems(const SortedPlan& p);
+cudaError_t launch_sorted_split(const SortedPlan& p, int64_t m, int64_t n, int64_t nnz, const int64_t* rp,
+                                const int32_t* col, const int32_t* order, const SortedScratch& w, cudaStream_t s);
+cudaError_t launch_sorted_move(const SortedPlan& p, int64_t m, int64_t n, int64_t nnz, const int32_t* col,
+                               const float* val, const SortedScratch& w, int64_t* cp, int32_t* trow, float* tval,
+                               cudaStream_t s);
+
 // Deterministic CSR -> CSC (rows ascending in the order `order`, or
 // natural order when null, within each column).  cnt holds B*n int32,
 // colcount n int64, scan_tmp scan_temp_elems(n) int64, bad one int32 that

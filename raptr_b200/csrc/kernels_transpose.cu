@@ -16,7 +16,8 @@
 // from column counts taken in the last pass's histogram.
 //
 // Scales as (passes x 3) streaming sweeps of the entries; used for matrices
-// whose columns fit two passes (n <= 2^20).  The first digit is 9 bits
+// whose columns fit two passes (n <= 2^20) and whose rows do not ascend, are sparse or
+// have fewer than 1025 columns (the others: kernels_transpose_sorted.cu).  The first digit is 9 bits
 // where the second (10 bits) still covers the column, so that a chunk of the
 // first scatter holds full 32-byte runs per digit.
 #include <algorithm>
