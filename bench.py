@@ -320,8 +320,7 @@ def synth_measurement(R, torch, ctx, w, lst, dist=None):
 def run_job(R, torch, ctx, w, lst, y_dev, dist=None):
     """One reconstruction job; returns per-phase device times (ms) and the
     device time of every forward and back pass of its iterations (CUDA
-    events between the passes, on the stream they are launched on: stream
-    launches, which run the iterations as fast as one CUDA graph of them)."""
+    events between the passes, on the stream they are launched on)."""
     g = w["geom"]
     ev = [torch.cuda.Event(enable_timing=True) for _ in range(5)]
     ev[0].record()
@@ -367,7 +366,7 @@ def precision_report(R, torch, ctx, w, lst, y_dev, peak):
     """The FP16-matrix form (plain: 6 bytes per entry; delta-coded: 4) beside
     the FP32 one, all against the FP64 iteration on the same matrix:
     relative L2 and max error of the image after 10 / 25 / 50 iterations,
-    iteration rates (CUDA graph) and the roofline of the FP16 passes."""
+    iteration rates and the roofline of the FP16 passes."""
     g = w["geom"]
     n = g.n_voxels
     A = ctx.build(lst, w["nrays"], SEED)
@@ -447,8 +446,7 @@ def batch_report(R, torch, ctx, w, lst, plain_iters_per_s, peak, n_frames=64, ni
     """The batched dynamic-PET form: n_frames frames sharing the matrix,
     activity x_true * exp(-k_j f) with per-voxel washout rates k ~ U[0.01,
     0.1] per frame, counts per frame log-uniform in [1e5, 1e8], solved
-    together with the FP16 matrix (frame tile from the autotuner, CUDA-graph
-    iterations).  Reports frame-iterations per second against the plain
+    together with the FP16 matrix (frame tile from the autotuner).  Reports frame-iterations per second against the plain
     FP32 single-frame rate, and frame 0's image against the FP64 iteration."""
     g = w["geom"]
     n = g.n_voxels

@@ -76,8 +76,7 @@ typedef struct raptr_matrix raptr_matrix;
 
 int raptr_abi_version(void);
 const char* raptr_last_error(void);
-/* Number of kernels this library has launched in this process (kernels
- * replayed from a CUDA graph included). */
+/* Number of kernels this library has launched in this process. */
 int64_t raptr_kernel_launches(void);
 
 /* No counterpart in the reference (it frees its buffers with cudaFree).
@@ -245,8 +244,7 @@ typedef struct raptr_mlem_opts {
                         * launches: a CUDA graph of them is slower at any size) */
   double* h_loglik;    /* optional: per-iteration Poisson log-likelihood (FP64)  */
   float* h_kernel_ms;  /* optional: 2*n_iter device times (ms) of the two passes of
-                          each iteration, from CUDA events on the stream; when
-                          set the loop is launched without a graph             */
+                          each iteration, from CUDA events on the stream       */
   const int32_t* d_row_rank; /* optional, with the transpose: the CSC's row
                           index is the position in an order, d_row_rank[row]
                           the row's position (raptr_matrix_row_order)         */

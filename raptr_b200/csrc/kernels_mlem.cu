@@ -1,11 +1,11 @@
 // CSR SpMV (forward and back projection), the MLEM element-wise operations
 // and the fused MLEM projection for sm_100a.
 //
-// All kernels here are HBM-bandwidth bound: the matrix streams once per
-// call with 16-byte vector loads (four columns + four values per lane), the
-// image x (a few MB) stays in L2, and back projection accumulates with
-// fire-and-forget float reductions (red.global.add.f32) into the image,
-// which is also L2-resident.
+// The matrix streams once per call, its lanes on consecutive entries; the image x
+// (a few MB) stays in L2.  The dot products by rows and by columns are HBM-bandwidth
+// bound.  Back projection by rows accumulates with fire-and-forget float
+// reductions (red.global.add.f32) into the image, which is also L2-resident;
+// L2 serves them per 32-byte sector, and they bound it.
 #include <algorithm>
 #include <cstdint>
 
