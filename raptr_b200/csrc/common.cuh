@@ -199,9 +199,16 @@ __device__ __forceinline__ bool row_cells(const DGeom& g, const Channel& ch, con
   const float rest = q - w * w;  // squared distance = rest + a2*dz^2 - 2*w*uz*dz
   *in0 = 0;
   *in1 = -1;
-  if (c.a2 < 1e-6f) {  // along z
+  if (c.a2 < 1e-6f) {  // along z: the squared distances of the row's voxels lie within +-s of each other
+    const float z0 = g.o[2] - ch.c0[2], z1 = z0 + float(nz) * g.d[2], D = fmaxf(fabsf(z0), fabsf(z1));
+    const float s = 2.f * fabsf(w) * D + c.a2 * D * D, m = margin + 4e-6f * s;
+    if (rest - s > c.r2 + m) return false;
     *lo = 0;
     *hi = nz - 1;
+    if (rest + s < c.r2 - m) {
+      *in0 = 0;
+      *in1 = nz - 1;
+    }
     return true;
   }
   const float B = w * c.uz, inv = 1.0f / c.a2;
