@@ -485,11 +485,13 @@ __device__ void sort_and_write(int* keys, float* vals, int total, int32_t* __res
 // A ray costs the same in any direction, while a walk takes one step per
 // crossing (75 at 0 degrees, ~110 at 45 for 70^3 voxels).  Measured against
 // the walk into dense windows with shared-memory atomics that it replaces:
-// 60,000 rows of 70^3 x 1000 rays 19.4 -> 13.5 ms, 12,345 rows of 100^3 x 999
-// rays 12.6 -> 5.1 ms (half of those rows did not fit the dense windows).
-// Main loop, ~54 issue slots per (ray, slab) and as many again for half of
+// 60,000 rows of 70^3 x 1000 rays 21.9 -> 12.4 ms, 12,345 rows of 100^3 x 999
+// rays 9.0 -> 4.1 ms (half of those rows did not fit the dense windows).
+// Main loop, ~50 issue slots per (ray, slab) and as many again for half of
 // the packed operations: 2/3 of the time; ray generation, set-up and
-// compaction the rest.
+// compaction the rest.  The ray's 112 bytes matter too: with 128 or 144 (to save
+// one operation per slab) three blocks no longer share an SM, or two rays' loads
+// their banks, and the kernel is 12 to 15 % slower.
 //
 // Exactness.  The plane parameters are computed with the operations of
 // walk_ray (and of the reference), so each is the same float.  A segment of
@@ -786,6 +788,14 @@ struct SlabShape {
   int batch = 0;  // rays staged at a time
   size_t smem() const { return size_t(acc_floats + stage_floats) * 4; }
 };
+constexpr int kMostSlots = 64, kMostStage = 8192;  // planned for: voxels of a slab's window, floats of a finished row
+// The most of any grid: the kernel's limit is always set to it, so that builds of
+// different grids on two threads do not set it below each other's need.
+constexpr int kSlabRayFloats = int(sizeof(SlabRay) / 4);
+constexpr int kSlabSmem =
+    ((kSlabs * kMostSlots + 3) * kSlabThreads +
+     (kSlabThreads * kSlabRayFloats > kMostStage ? kSlabThreads * kSlabRayFloats : kMostStage)) * 4;
+static_assert(kSlabSmem <= 220 * 1024, "fits a block");
 
 // One block per row.  The sums of the row's windows (per slab of A the
 // voxels [ulo, ulo+wu) x [vlo, vlo+wv) that the crystals' hull can reach)
@@ -938,7 +948,8 @@ __global__ void __launch_bounds__(kSlabThreads, kSlabBlocks)
       auto range = [&](int ax, float lo, float hi, int* first) {
         const int n = axis_n(g, ax);
         const float inv = __fdividef(1.0f, axis_d(g, ax));
-        const int a = int(floorf((lo - axis_o(g, ax)) * inv - 0.02f)), b = int(floorf((hi - axis_o(g, ax)) * inv + 0.02f));
+        const int a = int(floorf((lo - axis_o(g, ax)) * inv - 0.02f));
+        const int b = int(floorf((hi - axis_o(g, ax)) * inv + 0.02f));
         const int l = min(max(a, 0), n - 1);
         *first = l;
         return max(min(max(b, 0), n - 1) - l, 0) + 1;
@@ -1351,10 +1362,10 @@ SlabShape slab_shape(const DGeom& g, int nrays) {
     }
   }
   const double wy = g.segy / g.d[1] + 2.1, wh = 1.5 * g.segz / std::min(g.d[0], g.d[2]) + 2.1;
-  const int W = int(std::min(std::ceil(wy * wh), 64.0));
+  const int W = int(std::min(std::ceil(wy * wh), double(kMostSlots)));
   sh.acc_floats = (kSlabs * W + 3) * sh.threads;
   sh.batch = most;
-  sh.stage_floats = std::max(sh.batch * int(sizeof(SlabRay) / 4), std::min(50 * std::max(g.n[0], g.n[2]), 8192));
+  sh.stage_floats = std::max(sh.batch * kSlabRayFloats, std::min(50 * std::max(g.n[0], g.n[2]), kMostStage));
   return sh;
 }
 
@@ -1378,7 +1389,7 @@ cudaError_t launch_level(const DGeom& g, const float2* d_sincos, const int32_t* 
   }
   if (parts & 1) {
     const SlabShape sh = slab_shape(g, nrays);
-    e = cudaFuncSetAttribute(sm_slab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sh.smem()));
+    e = cudaFuncSetAttribute(sm_slab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabSmem);
     if (e != cudaSuccess) return e;
     sm_slab_kernel<<<unsigned(nrows), unsigned(sh.threads), sh.smem(), s>>>(
         g, d_sincos, d_cnl, row0, nrays, seed, H, sh.acc_floats, sh.stage_floats, sh.batch, st_col, st_val, row_nnz,
