@@ -1745,8 +1745,8 @@ raptr_status batch_args(raptr_ctx* ctx, int64_t m, int64_t n, int32_t K, int32_t
   return RAPTR_OK;
 }
 
-// The widest tile: 64 frames of 70^3 x 5.14M channels take 112 ms an iteration in
-// one tile of 64 and 120 in two of 32, of x 57,122 channels 1.53 and 1.92.
+// The widest tile: 64 frames of 70^3 x 5.14M channels take 105 ms an iteration in
+// one tile of 64 and 112 in two of 32, of x 57,122 channels 1.53 and 1.92.
 int default_frame_tile(int K) { return batch_tile_supported(K, 64) ? 64 : 0; }
 
 }  // namespace

@@ -505,7 +505,7 @@ void raptr_server::loop() {
         e->launch_error = "batch relayout failed";
       } else {
         // all frames in sweeps of at most 64 (a multiple of 4 frames): one
-        // 64-frame sweep takes 112 ms at 70^3, two of 32 take 120 ms
+        // 64-frame sweep takes 105 ms at 70^3, two of 32 take 112 ms
         e->launch_status = raptr_mlem_batch(e->ctx, e->m, e->n, e->K, 1, e->rp, e->col, e->hval, e->rscale, e->cp,
                                             e->trow, e->htval, e->rank, e->Y, e->s, e->X(), 1, 64, nullptr,
                                             e->stream);
