@@ -328,9 +328,10 @@ cudaError_t launch_tile(const BatchArgs& a, bool forward, int f0, double* acc, u
         a.m, a.K, f0, a.rp, a.col, static_cast<const VT*>(a.val), a.half ? a.rscale : nullptr, a.Y,
         compact ? a.Xt : a.X + f0, compact ? KT : a.K, a.rank, a.E + int64_t(f0) * a.m);
   } else {
-    // blocks for kColsPerWarp columns a warp, and enough to fill the GPU
+    // blocks for all columns at kColsPerWarp columns a warp (a warp takes no more),
+    // and enough to fill the GPU
     const int64_t per = kColsPerWarp * (kThreads / 32);
-    const int64_t blocks = std::min<int64_t>(std::max<int64_t>((a.n + per - 1) / per, 148 * 10), grid_warps(a.n));
+    const int64_t blocks = std::max<int64_t>((a.n + per - 1) / per, std::min<int64_t>(148 * 10, grid_warps(a.n)));
     batch_back_kernel<KT, VT><<<unsigned(blocks), kThreads, 0, s>>>(a.n, a.K, f0, next, a.cp, a.trow, static_cast<const VT*>(a.tval),
                                                   a.E + int64_t(f0) * a.m,
                                                   a.X, a.S, a.cols, a.n_full, a.XX, acc, grp.mode ? a.seg : nullptr,
