@@ -19,24 +19,66 @@ __device__ __forceinline__ int64_t column_unit(int64_t total) {
   return u < 2048 ? 2048 : u;
 }
 
-// Sums of four values over the warp: lane l gets that of value l / 8.
-__device__ __forceinline__ float warp_sum4(float s0, float s1, float s2, float s3, int lane) {
-  const bool h = (lane & 16) != 0, q = (lane & 8) != 0;
-  float a = (h ? s2 : s0) + __shfl_xor_sync(0xffffffffu, h ? s0 : s2, 16);
-  float b = (h ? s3 : s1) + __shfl_xor_sync(0xffffffffu, h ? s1 : s3, 16);
-  a = (q ? b : a) + __shfl_xor_sync(0xffffffffu, q ? a : b, 8);
-#pragma unroll
-  for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-  return a;
+// Neumaier compensated addition: (s, c) += v.
+__device__ __forceinline__ void two_sum_add(float& s, float& c, float v) {
+  const float t = s + v;
+  if (fabsf(s) >= fabsf(v))
+    c += (s - t) + v;
+  else
+    c += (v - t) + s;
+  s = t;
 }
 
-// Dot products of four columns of at most kShortColumn entries with e; lane l
-// gets that of column l / 8.  All loads of the four are in flight together.
-template <class VT, class F>
+// A sum in FP32: plain, or with its compensation (the FP16 form's).
+struct PlainSum {
+  float s = 0.f;
+  __device__ __forceinline__ void add(float v) { s += v; }
+  __device__ __forceinline__ void add(const PlainSum& o) { s += o.s; }
+  __device__ __forceinline__ PlainSum from_lane_xor(int o) const {
+    PlainSum r;
+    r.s = __shfl_xor_sync(0xffffffffu, s, o);
+    return r;
+  }
+  __device__ __forceinline__ float value() const { return s; }
+};
+struct CompensatedSum {
+  float s = 0.f, c = 0.f;
+  __device__ __forceinline__ void add(float v) { two_sum_add(s, c, v); }
+  __device__ __forceinline__ void add(const CompensatedSum& o) {
+    two_sum_add(s, c, o.s);
+    c += o.c;
+  }
+  __device__ __forceinline__ CompensatedSum from_lane_xor(int o) const {
+    CompensatedSum r;
+    r.s = __shfl_xor_sync(0xffffffffu, s, o);
+    r.c = __shfl_xor_sync(0xffffffffu, c, o);
+    return r;
+  }
+  __device__ __forceinline__ float value() const { return s + c; }
+};
+
+// Sums of four values over the warp: lane l gets that of value l / 8.
+template <class Sum>
+__device__ __forceinline__ float warp_sum4(const Sum (&s)[4], int lane) {
+  const bool h = (lane & 16) != 0, q = (lane & 8) != 0;
+  Sum a = h ? s[2] : s[0], b = h ? s[3] : s[1];
+  a.add((h ? s[0] : s[2]).from_lane_xor(16));
+  b.add((h ? s[1] : s[3]).from_lane_xor(16));
+  Sum t = q ? b : a;
+  t.add((q ? a : b).from_lane_xor(8));
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) t.add(t.from_lane_xor(o));
+  return t.value();
+}
+
+// Dot products of four columns of at most kShortColumn entries with e, in
+// sums of type Sum; lane l gets that of column l / 8.  All loads of the four are
+// in flight together.
+template <class Sum, class VT, class F>
 __device__ __forceinline__ float short_columns(const int32_t* __restrict__ trow, const VT* __restrict__ tval,
                                                const int64_t (&b)[4], const int (&len)[4],
                                                const float* __restrict__ e, int lane, F to_float) {
-  float s[4];
+  Sum s[4];
   int r[4][2];
   VT w[4][2];
 #pragma unroll
@@ -49,12 +91,11 @@ __device__ __forceinline__ float short_columns(const int32_t* __restrict__ trow,
     }
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    s[k] = 0.f;
 #pragma unroll
     for (int u = 0; u < 2; u++)
-      if (r[k][u] >= 0) s[k] += to_float(w[k][u]) * __ldg(e + r[k][u]);
+      if (r[k][u] >= 0) s[k].add(to_float(w[k][u]) * __ldg(e + r[k][u]));
   }
-  return warp_sum4(s[0], s[1], s[2], s[3], lane);
+  return warp_sum4(s, lane);
 }
 
 // c_j = <column j, e> for every column, by `dot(b, e)` (one column of any

@@ -69,16 +69,6 @@ __device__ __forceinline__ void block_add_d(double v, double* dst) {
 
 __device__ __forceinline__ float h2f(uint16_t h) { return __half2float(__ushort_as_half(h)); }
 
-// Neumaier compensated addition: (s, c) += v.
-__device__ __forceinline__ void two_sum_add(float& s, float& c, float v) {
-  const float t = s + v;
-  if (fabsf(s) >= fabsf(v))
-    c += (s - t) + v;
-  else
-    c += (v - t) + s;
-  s = t;
-}
-
 // ---- conversion ------------------------------------------------------------
 
 __global__ void __launch_bounds__(kThreads) half_rows_kernel(int64_t m, const int64_t* __restrict__ rp,
@@ -232,7 +222,7 @@ __device__ __forceinline__ float col_dot_half(const int32_t* __restrict__ trow, 
     two_sum_add(s, c, (f4.x * g8 + f4.y * g9) + (f5.x * g10 + f5.y * g11));
     two_sum_add(s, c, (f6.x * g12 + f6.y * g13) + (f7.x * g14 + f7.y * g15));
   }
-  // the rest as one step with predicated loads (see the FP32 row_dot)
+  // the rest as one step with predicated loads, all in flight together
   int4 r[4];
   uint2 w[4];
 #pragma unroll
@@ -287,8 +277,8 @@ __global__ void __launch_bounds__(kThreads, 4) mlem_back_half_kernel(int64_t n, 
   const double sum = back_columns<UPDATE>(
       n, cp, x, sens, out, next, [&](int64_t b, int64_t b1) { return col_dot_half(trow, htval, b, b1, e, lane); },
       [&](const int64_t(&b)[4], const int(&len)[4]) {
-        return short_columns(trow, reinterpret_cast<const unsigned short*>(htval), b, len, e, lane,
-                             [](unsigned short v) { return h2f(v); });
+        return short_columns<CompensatedSum>(trow, reinterpret_cast<const unsigned short*>(htval), b, len, e, lane,
+                                             [](unsigned short v) { return h2f(v); });
       });
   if (UPDATE) block_add_d(sum, acc);
 }
