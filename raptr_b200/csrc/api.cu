@@ -471,7 +471,7 @@ struct Builder {
           if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_flags + 2 + b, 0, sizeof(int32_t), P);
           if (e == cudaSuccess)
             e = launch_sm_rows(level, ctx->dg, ctx->d_sincos, d_cnl, r, k, nrays, seed, nullptr, st_col[b],
-                               st_val[b], row_nnz[b], ctx->d_flags + 2 + b, P, nullptr, kRowsTable);
+                               st_val[b], row_nnz[b], ctx->d_flags + 2 + b, P, ctx->d_flags + 4, kRowsTable);
           if (e == cudaSuccess)
             e = cudaMemcpyAsync(const_cast<int32_t*>(h_flags) + 2 + b, ctx->d_flags + 2 + b, sizeof(int32_t),
                                 cudaMemcpyDeviceToHost, P);

@@ -55,11 +55,11 @@ int sm_pick_level(const DGeom& g, int nrays);
 // Builds rows [row0, row0+nrows) of the list into staging slots (slot i at
 // st_col/st_val + i*capacity).  row_nnz[i] = entries, or -1 if the table
 // overflowed.  *d_flags |= 1 on overflow, |= 4 for a channel id out of range.
-// With d_table_reasons (4 ints) the rows the slab kernel leaves to the hash
-// table are counted by reason: no slab axis, windows over the slot limit,
-// a ray outside the windows, a slot decoding outside the grid.  parts: 1 =
-// the slab kernel only (rows it cannot take keep row_nnz = -2), 2 = the
-// table kernel for those rows only, 3 = both; with d_rays every row takes
+// With d_table_reasons (4 ints) the rows left to the hash table are counted by
+// reason: no slab axis, windows over the slot limit, a ray outside the windows,
+// a slot decoding outside the grid.  parts: 1 = the slab kernel only (rows it
+// cannot take keep row_nnz = -2 or -3), 2 = the window and table kernels for
+// those rows only, 3 = all; with d_rays every row takes
 // the table kernel whatever parts says.
 constexpr int kRowsDense = 1, kRowsTable = 2, kRowsAll = 3;
 cudaError_t launch_sm_rows(int level, const DGeom& g, const float2* d_sincos, const int32_t* d_cnl, int64_t row0,

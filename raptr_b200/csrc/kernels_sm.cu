@@ -12,8 +12,10 @@
 //      the entry parameters, masked min of the exit parameters, and
 //      (exit - entry) * |end - start|.  When the two crystals lie on opposite
 //      sides of the grid along x or z, threads own slabs of the grid
-//      (sm_slab_kernel); the other rows walk each ray from plane to plane into
-//      an open-addressing hash table keyed by voxel id (sm_table_kernel);
+//      (sm_slab_kernel); where the slabs' windows are too large for that
+//      (crystals of many voxels) each ray is walked from plane to plane into
+//      the windows (sm_window_kernel); the other rows walk their rays into an
+//      open-addressing hash table keyed by voxel id (sm_table_kernel);
 //   3. the sums are compacted keeping voxels that pass the exact cylinder
 //      test (the reference only evaluates candidates,
 //      src/getSystemMatrixDeviceOnly.cu:433-470), put in voxel-id order,
@@ -117,6 +119,42 @@ struct KeyIndex {
   __device__ __forceinline__ void set(int i0, int i1, int i2) { key = i0 * nyz + i1 * nz + i2; }
   __device__ __forceinline__ void advance(bool ax, bool ay) { key += ax ? k0 : (ay ? k1 : k2); }
   __device__ __forceinline__ void add(float L) const { table->add(key, L); }
+};
+
+// The same into the windows of a row with slab axis A (x or z): slot
+// base[s] + iu * wv + iv for a voxel of slab s, which a step along A moves by
+// dk[s] more than (u, v) do; no key is stored or compared.
+template <int A>
+struct WindowIndex {
+  float* sums;
+  const int* base;
+  const int* dk;
+  int wv, nslots;
+  int slot, sa, ka, sta, ku, kv;
+  __device__ __forceinline__ void begin(const int step[3]) {
+    sta = step[A];
+    ku = step[A == 0 ? 1 : 0] * wv;
+    kv = step[A == 0 ? 2 : 1];
+  }
+  __device__ __forceinline__ void set(int i0, int i1, int i2) {
+    sa = A == 0 ? i0 : i2;
+    slot = A == 0 ? base[i0] + i1 * wv + i2 : base[i2] + i0 * wv + i1;
+    ka = dk[sa];
+  }
+  __device__ __forceinline__ void advance(bool ax, bool ay) {
+    if (A == 0) {
+      slot += ax ? ka : (ay ? ku : kv);
+      sa = ax ? sa + sta : sa;
+    } else {
+      slot += ax ? ku : (ay ? kv : ka);
+      sa = (ax || ay) ? sa : sa + sta;
+    }
+    ka = dk[sa];
+  }
+  // a slot outside the windows is the spare one, which the row looks at afterwards
+  __device__ __forceinline__ void add(float L) const {
+    atomicAdd(&sums[unsigned(slot) < unsigned(nslots) ? slot : nslots], L);
+  }
 };
 
 // Visits every grid voxel whose intersection length with ray r is positive.
@@ -771,9 +809,9 @@ __device__ __forceinline__ bool slab_ray(const DGeom& g, const float r[6], int A
 __device__ __forceinline__ unsigned div_magic(int d) { return 0xffffffffu / unsigned(d) + 1u; }
 __device__ __forceinline__ int div_by(int i, int d, unsigned m) { return d == 1 ? i : int(__umulhi(unsigned(i), m)); }
 
-// Row status the slab kernel leaves for the table kernel: the row is to be
-// built with the hash table.
-constexpr int kRowToTable = -2;
+// Row status the slab kernel leaves: the row is to be built with the hash
+// table, or by walks into its windows, which are too large for the slab kernel.
+constexpr int kRowToTable = -2, kRowToWindows = -3;
 
 constexpr int kMaxSlabs = 256;
 
@@ -786,6 +824,7 @@ struct SlabShape {
   int acc_floats = 0;
   int stage_floats = 0;
   int batch = 0;  // rays staged at a time
+  bool large_windows = false;  // some rows' windows may not fit
   size_t smem() const { return size_t(acc_floats + stage_floats) * 4; }
 };
 constexpr int kMostSlots = 64, kMostStage = 8192;  // planned for: voxels of a slab's window, floats of a finished row
@@ -797,13 +836,83 @@ constexpr int kSlabSmem =
      (kSlabThreads * kSlabRayFloats > kMostStage ? kSlabThreads * kSlabRayFloats : kMostStage)) * 4;
 static_assert(kSlabSmem <= 220 * 1024, "fits a block");
 
+// A row's crystals: boxes rotated about y, four corners in (x, z), two bounds in y.
+struct Crystals {
+  float x[2][4], z[2][4], y[2][2];
+};
+
+// The slab axis: of x and z, the one along which the crystals lie on opposite
+// sides of the grid, the channel's dominant direction first; -1 if none.  *sdir =
+// the rays' direction along it.
+__device__ __forceinline__ int slab_axis(const DGeom& g, const float ab[3], const Crystals& c, int* sdir) {
+  *sdir = 0;
+  const int first = fabsf(ab[0]) >= fabsf(ab[2]) ? 0 : 2;
+  for (int k = 0; k < 2; k++) {
+    const int a = k == 0 ? first : 2 - first;
+    if (axis_n(g, a) > kMaxSlabs) continue;
+    const float* p = a == 0 ? c.x[0] : c.z[0];
+    const float* q = a == 0 ? c.x[1] : c.z[1];
+    const float plo = fminf(fminf(p[0], p[1]), fminf(p[2], p[3])), phi = fmaxf(fmaxf(p[0], p[1]), fmaxf(p[2], p[3]));
+    const float qlo = fminf(fminf(q[0], q[1]), fminf(q[2], q[3])), qhi = fmaxf(fmaxf(q[0], q[1]), fmaxf(q[2], q[3]));
+    const float c0 = axis_o(g, a), c1 = axis_o(g, a) + float(axis_n(g, a)) * axis_d(g, a);
+    const float m = 1e-6f * (1.0f + fabsf(c0) + fabsf(c1));
+    if (phi + m < c0 && qlo - m > c1) *sdir = 1;
+    if (qhi + m < c0 && plo - m > c1) *sdir = -1;
+    if (*sdir != 0) return a;
+  }
+  return -1;
+}
+
+// The window of slab sl of axis A: the first voxel and the number of voxels along
+// u and v that the crystals' hull reaches at the slab's two faces, with `margin`
+// voxels on each side.
+__device__ __forceinline__ void slab_window(const DGeom& g, const Crystals& c, int A, int sl, float margin, int* u0,
+                                            int* nu, int* v0, int* nv) {
+  const float* pa = A == 0 ? c.x[0] : c.z[0];
+  const float* qa = A == 0 ? c.x[1] : c.z[1];
+  const float* pw = A == 0 ? c.z[0] : c.x[0];
+  const float* qw = A == 0 ? c.z[1] : c.x[1];
+  const float c0 = axis_o(g, A) + float(sl) * axis_d(g, A), c1 = axis_o(g, A) + float(sl + 1) * axis_d(g, A);
+  float wlo = INFINITY, whi = -INFINITY, tlo = INFINITY, thi = -INFINITY;
+#pragma unroll 4
+  for (int ij = 0; ij < 16; ij++) {
+    const int i = ij >> 2, j = ij & 3;
+    const float inv = __fdividef(1.0f, qa[j] - pa[i]);
+    const float t0 = (c0 - pa[i]) * inv, t1 = (c1 - pa[i]) * inv;
+    const float w0 = pw[i] + t0 * (qw[j] - pw[i]), w1 = pw[i] + t1 * (qw[j] - pw[i]);
+    wlo = fminf(wlo, fminf(w0, w1));
+    whi = fmaxf(whi, fmaxf(w0, w1));
+    tlo = fminf(tlo, fminf(t0, t1));
+    thi = fmaxf(thi, fmaxf(t0, t1));
+  }
+  const float dy0 = c.y[1][0] - c.y[0][0], dy1 = c.y[1][1] - c.y[0][1];
+  const float ylo = c.y[0][0] + fminf(tlo * dy0, thi * dy0);
+  const float yhi = c.y[0][1] + fmaxf(tlo * dy1, thi * dy1);
+  auto range = [&](int ax, float lo, float hi, int* first) {
+    const int n = axis_n(g, ax);
+    const float inv = __fdividef(1.0f, axis_d(g, ax));
+    const int a = int(floorf((lo - axis_o(g, ax)) * inv - margin));
+    const int b = int(floorf((hi - axis_o(g, ax)) * inv + margin));
+    const int l = min(max(a, 0), n - 1);
+    *first = l;
+    return max(min(max(b, 0), n - 1) - l, 0) + 1;
+  };
+  int y0, w0;
+  const int ny = range(1, ylo, yhi, &y0);
+  const int nw = range(A == 0 ? 2 : 0, wlo, whi, &w0);
+  *u0 = A == 0 ? y0 : w0;
+  *nu = A == 0 ? ny : nw;
+  *v0 = A == 0 ? w0 : y0;
+  *nv = A == 0 ? nw : ny;
+}
+
 // One block per row.  The sums of the row's windows (per slab of A the
 // voxels [ulo, ulo+wu) x [vlo, vlo+wv) that the crystals' hull can reach)
 // are kept per thread: slot w of thread t at acc[w * S + t], S = the threads
 // in use rounded up to a warp.  A row with more slots per slab than fit runs
-// with fewer groups of rays; one whose slots do not fit one group, that has
-// no slab axis, or one of whose rays needs the general walk gets row_nnz =
-// kRowToTable and is built by sm_table_kernel.
+// with fewer groups of rays; one whose slots do not fit one group gets row_nnz =
+// kRowToWindows, one that has no slab axis or one of whose rays needs the general
+// walk kRowToTable.
 //
 // The windows hold every voxel a ray visits: a ray lies in the convex hull
 // of the two crystals, the windows are the hull's extents at the slab's two
@@ -823,7 +932,7 @@ __global__ void __launch_bounds__(kSlabThreads, kSlabBlocks)
   SlabRay* rays = reinterpret_cast<SlabRay*>(stage);
   __shared__ Channel ch;
   __shared__ int bad_walk, to_table, outside, win_u, win_v;
-  __shared__ float corner_x[2][4], corner_z[2][4], corner_y[2][2];
+  __shared__ Crystals cr;
   __shared__ int warp_sums[32];
   __shared__ short ulo[kMaxSlabs], vlo[kMaxSlabs];
   __shared__ int zbox[4];
@@ -839,8 +948,8 @@ __global__ void __launch_bounds__(kSlabThreads, kSlabBlocks)
   }
   auto table = [&](int why) {  // called by every thread, or by one
     if (tid == 0) {
-      row_nnz[blockIdx.x] = kRowToTable;
-      if (reasons) atomicAdd(reasons + why, 1);
+      row_nnz[blockIdx.x] = why == 1 ? kRowToWindows : kRowToTable;
+      if (reasons && why != 1) atomicAdd(reasons + why, 1);
     }
   };
   if (warp == 0) {
@@ -857,9 +966,9 @@ __global__ void __launch_bounds__(kSlabThreads, kSlabBlocks)
     trafo_apply(m, float(c & 1), float(c >> 1), float(c >> 1), p);
     trafo_apply(m, 0.5f, 0.5f, 0.5f, mid);
     if (lane < 8) {
-      corner_x[b][c] = p[0];
-      corner_z[b][c] = p[2];
-      if ((c & 1) == 0) corner_y[b][c >> 1] = p[1];
+      cr.x[b][c] = p[0];
+      cr.z[b][c] = p[2];
+      if ((c & 1) == 0) cr.y[b][c >> 1] = p[1];
     }
     if (lane < 8 && c == 0) {
       float* to = b == 0 ? ch.m0 : ch.m1;
@@ -893,25 +1002,8 @@ __global__ void __launch_bounds__(kSlabThreads, kSlabBlocks)
     ch.abs_ab = norm3_exact(ch.ab[0], ch.ab[1], ch.ab[2]);
     ch.radius = RFMUL(0.5f, RFADD(norm3_exact(g.d[0], g.d[1], g.d[2]), norm3_exact(g.segx, g.segy, g.segz)));
   }
-  // the slab axis: of x and z, the one along which the crystals lie on
-  // opposite sides of the grid, the channel's dominant direction first
-  int A = -1, sdir = 0;
-  {
-    const int first = fabsf(ch.ab[0]) >= fabsf(ch.ab[2]) ? 0 : 2;
-    for (int k = 0; k < 2 && A < 0; k++) {
-      const int a = k == 0 ? first : 2 - first;
-      if (axis_n(g, a) > kMaxSlabs) continue;
-      const float* p = a == 0 ? corner_x[0] : corner_z[0];
-      const float* q = a == 0 ? corner_x[1] : corner_z[1];
-      const float plo = fminf(fminf(p[0], p[1]), fminf(p[2], p[3])), phi = fmaxf(fmaxf(p[0], p[1]), fmaxf(p[2], p[3]));
-      const float qlo = fminf(fminf(q[0], q[1]), fminf(q[2], q[3])), qhi = fmaxf(fmaxf(q[0], q[1]), fmaxf(q[2], q[3]));
-      const float c0 = axis_o(g, a), c1 = axis_o(g, a) + float(axis_n(g, a)) * axis_d(g, a);
-      const float m = 1e-6f * (1.0f + fabsf(c0) + fabsf(c1));
-      if (phi + m < c0 && qlo - m > c1) sdir = 1;
-      if (qhi + m < c0 && plo - m > c1) sdir = -1;
-      if (sdir != 0) A = a;
-    }
-  }
+  int sdir;
+  const int A = slab_axis(g, ch.ab, cr, &sdir);
   if (A < 0) {
     table(0);
     return;
@@ -925,42 +1017,12 @@ __global__ void __launch_bounds__(kSlabThreads, kSlabBlocks)
   {
     int wu_max = 0, wv_max = 0;
     for (int sl = tid; sl < na; sl += T) {
-      const float* pa = A == 0 ? corner_x[0] : corner_z[0];
-      const float* qa = A == 0 ? corner_x[1] : corner_z[1];
-      const float* pw = A == 0 ? corner_z[0] : corner_x[0];
-      const float* qw = A == 0 ? corner_z[1] : corner_x[1];
-      const float c0 = axis_o(g, A) + float(sl) * axis_d(g, A), c1 = axis_o(g, A) + float(sl + 1) * axis_d(g, A);
-      float wlo = INFINITY, whi = -INFINITY, tlo = INFINITY, thi = -INFINITY;
-#pragma unroll 4
-      for (int ij = 0; ij < 16; ij++) {
-        const int i = ij >> 2, j = ij & 3;
-        const float inv = __fdividef(1.0f, qa[j] - pa[i]);
-        const float t0 = (c0 - pa[i]) * inv, t1 = (c1 - pa[i]) * inv;
-        const float w0 = pw[i] + t0 * (qw[j] - pw[i]), w1 = pw[i] + t1 * (qw[j] - pw[i]);
-        wlo = fminf(wlo, fminf(w0, w1));
-        whi = fmaxf(whi, fmaxf(w0, w1));
-        tlo = fminf(tlo, fminf(t0, t1));
-        thi = fmaxf(thi, fmaxf(t0, t1));
-      }
-      const float dy0 = corner_y[1][0] - corner_y[0][0], dy1 = corner_y[1][1] - corner_y[0][1];
-      const float ylo = corner_y[0][0] + fminf(tlo * dy0, thi * dy0);
-      const float yhi = corner_y[0][1] + fmaxf(tlo * dy1, thi * dy1);
-      auto range = [&](int ax, float lo, float hi, int* first) {
-        const int n = axis_n(g, ax);
-        const float inv = __fdividef(1.0f, axis_d(g, ax));
-        const int a = int(floorf((lo - axis_o(g, ax)) * inv - 0.02f));
-        const int b = int(floorf((hi - axis_o(g, ax)) * inv + 0.02f));
-        const int l = min(max(a, 0), n - 1);
-        *first = l;
-        return max(min(max(b, 0), n - 1) - l, 0) + 1;
-      };
-      int y0, w0;
-      const int ny = range(1, ylo, yhi, &y0);
-      const int nw = range(A == 0 ? 2 : 0, wlo, whi, &w0);
-      wu_max = max(wu_max, A == 0 ? ny : nw);
-      wv_max = max(wv_max, A == 0 ? nw : ny);
-      ulo[sl] = short(A == 0 ? y0 : w0);
-      vlo[sl] = short(A == 0 ? w0 : y0);
+      int u0, nu, v0, nv;
+      slab_window(g, cr, A, sl, 0.02f, &u0, &nu, &v0, &nv);
+      wu_max = max(wu_max, nu);
+      wv_max = max(wv_max, nv);
+      ulo[sl] = short(u0);
+      vlo[sl] = short(v0);
     }
     wu_max = __reduce_max_sync(0xffffffffu, wu_max);
     wv_max = __reduce_max_sync(0xffffffffu, wv_max);
@@ -1196,20 +1258,222 @@ __global__ void __launch_bounds__(kSlabThreads, kSlabBlocks)
   if (tid == 0) row_nnz[blockIdx.x] = total;
 }
 
+// Blocks per SM the window kernel is compiled for: what its shared memory leaves.
+constexpr int rest_blocks(int H) { return H <= 2048 ? 8 : (H <= 4096 ? 4 : (H <= 8192 ? 3 : 1)); }
+
+// Sums of a row that is walked into its windows: what leaves four blocks per SM
+// their registers' share at H <= 4096, and no less than the entries take that are
+// sorted in their place.
+__host__ __device__ constexpr int window_floats(int H) { return H <= 4096 ? 3 * H : 2 * H; }
+
+// Window kernel: the rows the slab kernel left for their windows' size
+// (kRowToWindows).  A row's rays are walked, thread by thread, into one array of
+// the windows' sums, by shared-memory atomics; a row that does not fit either, or one
+// of whose rays leaves its windows, is left to the table kernel.  The windows have a
+// margin of a voxel, since there is no bound eps on a ray's roundings here.  Bound by the
+// walks' instructions and the atomics, as the slab kernel's forerunner was, but with no
+// keys to look for: 4,000 rows x 300 rays of 70^3 voxels of 0.7 mm take 4.1 ms, with the
+// table kernel 6.4; 100^3 of 1.5 mm seen by 8 mm crystals 3.5 and 5.2.
+template <int H, int T, bool OISO>
+__global__ void __launch_bounds__(T, rest_blocks(H))
+    sm_window_kernel(DGeom g, const float2* __restrict__ sincos, const int32_t* __restrict__ cnl_ids, int64_t row0,
+                     int64_t nrows, int nrays, uint32_t seed, int32_t* __restrict__ st_col,
+                     float* __restrict__ st_val, int32_t* __restrict__ row_nnz, int32_t* __restrict__ flags,
+                     int32_t* __restrict__ reasons) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  float* sums = reinterpret_cast<float*>(smem);  // slots of the windows and the spare one
+  __shared__ Channel ch;
+  __shared__ Crystals cr;
+  __shared__ int bad_walk, to_table, outside, win_u, win_v;
+  __shared__ int warp_sums[32];
+  __shared__ int ulo[kMaxSlabs], vlo[kMaxSlabs], base[kMaxSlabs], dk[kMaxSlabs];
+  constexpr int NW = T / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nz = g.n[2], nyz = g.n[1] * nz;
+  for (int64_t bi = blockIdx.x; bi < nrows; bi += gridDim.x) {
+    if (row_nnz[bi] != kRowToWindows) continue;
+    // (called by every thread)
+    auto error = [&](int flag) {
+      if (tid == 0) {
+        row_nnz[bi] = -1;
+        atomicOr(flags, flag);
+      }
+    };
+    auto table = [&](int why) {
+      if (tid == 0) {
+        row_nnz[bi] = kRowToTable;
+        if (reasons) atomicAdd(reasons + why, 1);
+      }
+    };
+    const int cnl = cnl_ids[row0 + bi];  // in range: the slab kernel has looked
+    __syncthreads();                     // the previous row's use of the shared memory is over
+    if (tid == 0) {
+      channel_setup(g, sincos, cnl, ch);
+      bad_walk = to_table = outside = win_u = win_v = 0;
+    }
+    __syncthreads();
+    if (tid < 8) {
+      const int b = tid >> 2, c = tid & 3;
+      float p[3];
+      trafo_apply(b == 0 ? ch.m0 : ch.m1, float(c & 1), float(c >> 1), float(c >> 1), p);
+      cr.x[b][c] = p[0];
+      cr.z[b][c] = p[2];
+      if ((c & 1) == 0) cr.y[b][c >> 1] = p[1];
+    }
+    __syncthreads();
+    int sdir;
+    const int A = slab_axis(g, ch.ab, cr, &sdir);
+    if (A < 0) {
+      table(0);
+      continue;
+    }
+    const int na = axis_n(g, A);
+    for (int sl = tid; sl < na; sl += T) {
+      int u0, nu, v0, nv;
+      slab_window(g, cr, A, sl, 1.0f, &u0, &nu, &v0, &nv);
+      ulo[sl] = u0;
+      vlo[sl] = v0;
+      atomicMax(&win_u, nu);
+      atomicMax(&win_v, nv);
+    }
+    __syncthreads();
+    const int wu = win_u, wv = win_v, W = wu * wv;
+    if ((long long)na * wu * wv >= (long long)window_floats(H)) {
+      table(1);
+      continue;
+    }
+    const int nslots = na * W;
+    for (int sl = tid; sl < na; sl += T) {
+      auto at = [&](int k) { return k * W - ulo[k] * wv - vlo[k]; };
+      const int next = sdir > 0 ? sl + 1 : sl - 1;
+      base[sl] = at(sl);
+      dk[sl] = next >= 0 && next < na ? at(next) - at(sl) : 0;
+    }
+    for (int i = tid; i <= nslots; i += T) sums[i] = 0.f;
+    __syncthreads();
+
+    auto emit = [&](int ix, int iy, int iz, float L) {
+      const int s = A == 0 ? ix : iz;
+      const int u = (A == 0 ? iy : ix) - ulo[s], v = (A == 0 ? iz : iy) - vlo[s];
+      if (unsigned(u) < unsigned(wu) && unsigned(v) < unsigned(wv))
+        atomicAdd(&sums[s * W + u * wv + v], L);
+      else
+        to_table = 1;
+    };
+    // start offsets: the thread index bit-reversed, so that neighbouring lanes
+    // start far apart along the ray
+    const int part = int(__brev(threadIdx.x) >> 24);
+    auto walk = [&](auto index) {
+      for (int ray = tid; ray < nrays; ray += T) {
+        float r[6];
+        make_ray(ch, seed, cnl, ray, r);
+        const float da = A == 0 ? RFSUB(r[3], r[0]) : RFSUB(r[5], r[2]);
+        // (the voxels of a ray parallel to an axis's planes: the table kernel's threads share them)
+        if (!(sdir > 0 ? da > 0.f : da < 0.f) || r[0] == r[3] || r[1] == r[4] || r[2] == r[5]) {
+          to_table = 1;
+          break;
+        }
+        walk_ray<OISO>(g, ch, r, part, emit, index, &bad_walk, 0, 1);
+      }
+    };
+    if (A == 0)
+      walk(WindowIndex<0>{sums, base, dk, wv, nslots});
+    else
+      walk(WindowIndex<2>{sums, base, dk, wv, nslots});
+    __syncthreads();
+    if (bad_walk) {
+      error(2);
+      continue;
+    }
+    if (to_table || sums[nslots] != 0.f) {
+      table(2);
+      continue;
+    }
+
+    // each warp takes a run of slots: count those that are voxels of the row, clear
+    // the others, and after a scan of the counts write them
+    const int seg = ((nslots + NW - 1) / NW + 31) & ~31;
+    const int b0 = min(warp * seg, nslots), b1 = min(b0 + seg, nslots);
+    auto voxel = [&](int slot, int* x, int* y, int* z) {
+      const int s = slot / W, u = (slot - s * W) / wv;
+      const int iu = ulo[s] + u, iv = vlo[s] + (slot - s * W - u * wv);
+      *x = A == 0 ? s : iu;
+      *y = A == 0 ? iu : iv;
+      *z = A == 0 ? iv : s;
+    };
+    int cnt = 0;
+    for (int b = b0 + lane; b - lane < b1; b += 32) {
+      bool keep = false;
+      if (b < b1 && sums[b] > 0.f) {
+        int x, y, z;
+        voxel(b, &x, &y, &z);
+        if (x < g.n[0] && y < g.n[1] && z < g.n[2])
+          keep = candidate_test(g, ch, x, y, z);
+        else
+          outside = 1;
+        if (!keep) sums[b] = 0.f;
+      }
+      cnt += __popc(__ballot_sync(0xffffffffu, keep));
+    }
+    if (lane == 0) warp_sums[warp] = cnt;
+    __syncthreads();
+    if (outside) {
+      table(3);
+      continue;
+    }
+    int before = 0, total = 0;
+    for (int k = 0; k < NW; k++) {
+      before += k < warp ? warp_sums[k] : 0;
+      total += warp_sums[k];
+    }
+    if (total > H) {
+      error(1);
+      continue;
+    }
+    const float fr = float(nrays);
+    const size_t out = size_t(bi) * H;
+    for (int b = b0 + lane; b - lane < b1; b += 32) {
+      const bool keep = b < b1 && sums[b] > 0.f;
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      if (keep) {
+        const int pos = before + __popc(m & ((1u << lane) - 1u));
+        int x, y, z;
+        voxel(b, &x, &y, &z);
+        st_col[out + pos] = x * nyz + y * nz + z;
+        st_val[out + pos] = RFDIV(sums[b], fr);
+      }
+      before += __popc(m);
+    }
+    if (A == 0) {  // slab by slab, then y, z: column order
+      if (tid == 0) row_nnz[bi] = total;
+      continue;
+    }
+    int* keys = reinterpret_cast<int*>(smem);
+    float* vals = reinterpret_cast<float*>(keys + H);
+    __syncthreads();  // the sums are done with, the entries written
+    for (int i = tid; i < total; i += T) {
+      keys[i] = st_col[out + i];
+      vals[i] = st_val[out + i];
+    }
+    __syncthreads();
+    sort_and_write<T>(keys, vals, total, st_col, st_val, out, row_nnz + bi);
+  }
+}
+
 // Table kernel: its rays (generated, or given in `rays`) summed per voxel in
 // an open-addressing hash table of H keys in shared memory, then the voxels
 // with a positive sum that pass the cylinder test sorted into column order.
 // Each CTA takes rows blockIdx.x, blockIdx.x + gridDim.x, ... of the nrows.
-// With only_flagged it builds only the rows the slab kernel left with
-// kRowToTable and leaves the others alone (launched then with a small grid:
-// most workloads leave none, and the blocks only read the row states).
+// With only_flagged it builds only the rows the other kernels left and leaves
+// the others alone (launched then with a small grid: most workloads leave none,
+// and the blocks only read the row states).
 template <int H, int T, bool OISO>
 __global__ void __launch_bounds__(T) sm_table_kernel(DGeom g, const float2* __restrict__ sincos,
                                                      const int32_t* __restrict__ cnl_ids, int64_t row0, int64_t nrows,
                                                      int nrays, uint32_t seed, const float* __restrict__ rays,
                                                      int32_t* __restrict__ st_col, float* __restrict__ st_val,
                                                      int32_t* __restrict__ row_nnz, int32_t* __restrict__ flags,
-                                                     int only_flagged) {
+                                                     int32_t* __restrict__ reasons, int only_flagged) {
   extern __shared__ __align__(16) unsigned char smem[];
   int* keys = reinterpret_cast<int*>(smem);
   float* vals = reinterpret_cast<float*>(smem + H * sizeof(int));
@@ -1226,7 +1490,8 @@ __global__ void __launch_bounds__(T) sm_table_kernel(DGeom g, const float2* __re
   const int nyz = g.n[1] * g.n[2];
   const int nz = g.n[2];
   for (int64_t bi = blockIdx.x; bi < nrows; bi += gridDim.x) {
-    if (only_flagged && row_nnz[bi] != kRowToTable) continue;
+    const int state = only_flagged ? row_nnz[bi] : kRowToTable;
+    if (state > kRowToTable) continue;
     const int64_t li = row0 + bi;
     const int cnl = cnl_ids[li];
     if (cnl < 0 || cnl >= num_channels(g)) {
@@ -1242,6 +1507,7 @@ __global__ void __launch_bounds__(T) sm_table_kernel(DGeom g, const float2* __re
       overflow = 0;
       bad_walk = 0;
       n_parallel = 0;
+      if (reasons && state == kRowToWindows) atomicAdd(reasons + 1, 1);
     }
     for (int i = tid; i < H; i += T) {
       keys[i] = -1;
@@ -1366,6 +1632,14 @@ SlabShape slab_shape(const DGeom& g, int nrays) {
   sh.acc_floats = (kSlabs * W + 3) * sh.threads;
   sh.batch = most;
   sh.stage_floats = std::max(sh.batch * kSlabRayFloats, std::min(50 * std::max(g.n[0], g.n[2]), kMostStage));
+  // The largest windows are up to 1.7 times wy * wh (100^3 of 1.5 mm: no row of 49
+  // slots and more of 29).  Where they surely fit, the window kernel's launch is
+  // saved (2 us); a row that does not fit all the same takes the hash table.
+  for (int a = 0; a < 3; a += 2) {
+    const int nt = (g.n[a] + kSlabs - 1) / kSlabs, S = (nt + 31) & ~31;
+    const double fit = std::min(double(sh.stage_floats) / g.n[a], (double(sh.acc_floats) / S - 3) / kSlabs);
+    sh.large_windows = sh.large_windows || 1.7 * wy * wh > fit;
+  }
   return sh;
 }
 
@@ -1383,12 +1657,12 @@ cudaError_t launch_level(const DGeom& g, const float2* d_sincos, const int32_t* 
   if (d_rays) {
     // caller-supplied rays: the table builds every row, one CTA each
     table<<<unsigned(nrows), T, table_smem, s>>>(g, d_sincos, d_cnl, row0, nrows, nrays, seed, d_rays, st_col,
-                                                  st_val, row_nnz, d_flags, 0);
+                                                  st_val, row_nnz, d_flags, nullptr, 0);
     note_launches(1);
     return cudaGetLastError();
   }
+  const SlabShape sh = slab_shape(g, nrays);
   if (parts & 1) {
-    const SlabShape sh = slab_shape(g, nrays);
     e = cudaFuncSetAttribute(sm_slab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabSmem);
     if (e != cudaSuccess) return e;
     sm_slab_kernel<<<unsigned(nrows), unsigned(sh.threads), sh.smem(), s>>>(
@@ -1397,12 +1671,21 @@ cudaError_t launch_level(const DGeom& g, const float2* d_sincos, const int32_t* 
     note_launches(1);
   }
   if (parts & 2) {
-    // the rows the slab kernel left to the table (a few per million on
-    // the centred-cube workloads), four blocks per SM looking through the
-    // row states
+    // the rows the slab kernel left (a few per million on the centred-cube
+    // workloads), four blocks per SM looking through the row states
     const int64_t tb = std::min<int64_t>(nrows, 148 * 4);
+    if (sh.large_windows) {
+      auto window = oiso ? sm_window_kernel<H, T, true> : sm_window_kernel<H, T, false>;
+      const size_t smem = size_t(window_floats(H)) * 4;
+      static_assert(window_floats(H) >= 2 * H, "holds the entries to be sorted");
+      e = cudaFuncSetAttribute(window, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+      if (e != cudaSuccess) return e;
+      window<<<unsigned(tb), T, smem, s>>>(g, d_sincos, d_cnl, row0, nrows, nrays, seed, st_col, st_val, row_nnz,
+                                           d_flags, d_reasons);
+      note_launches(1);
+    }
     table<<<unsigned(tb), T, table_smem, s>>>(g, d_sincos, d_cnl, row0, nrows, nrays, seed, nullptr, st_col,
-                                              st_val, row_nnz, d_flags, 1);
+                                              st_val, row_nnz, d_flags, d_reasons, 1);
     note_launches(1);
   }
   return cudaGetLastError();
