@@ -1258,7 +1258,9 @@ __global__ void __launch_bounds__(kSlabThreads, kSlabBlocks)
   if (tid == 0) row_nnz[blockIdx.x] = total;
 }
 
-// Blocks per SM the window kernel is compiled for: what its shared memory leaves.
+// Blocks per SM the window and table kernels are compiled for: what their shared
+// memory leaves (at H = 8192 the table kernel alone took 99 registers, two blocks:
+// 4,000 rows x 300 of the caller's rays, 100^3 of 1.5 mm, 2.3 ms; so 1.75).
 constexpr int rest_blocks(int H) { return H <= 2048 ? 8 : (H <= 4096 ? 4 : (H <= 8192 ? 3 : 1)); }
 
 // Sums of a row that is walked into its windows: what leaves four blocks per SM
@@ -1468,7 +1470,7 @@ __global__ void __launch_bounds__(T, rest_blocks(H))
 // the others alone (launched then with a small grid: most workloads leave none,
 // and the blocks only read the row states).
 template <int H, int T, bool OISO>
-__global__ void __launch_bounds__(T) sm_table_kernel(DGeom g, const float2* __restrict__ sincos,
+__global__ void __launch_bounds__(T, rest_blocks(H)) sm_table_kernel(DGeom g, const float2* __restrict__ sincos,
                                                      const int32_t* __restrict__ cnl_ids, int64_t row0, int64_t nrows,
                                                      int nrays, uint32_t seed, const float* __restrict__ rays,
                                                      int32_t* __restrict__ st_col, float* __restrict__ st_val,
@@ -1528,27 +1530,25 @@ __global__ void __launch_bounds__(T) sm_table_kernel(DGeom g, const float2* __re
           make_ray(ch, seed, cnl, ray, r);
         }
       };
-      for (int ray = tid; ray < nrays; ray += T) {
-        float r[6];
-        ray_ends(ray, r);
-        if (r[0] == r[3] || r[1] == r[4] || r[2] == r[5]) {
-          const int at = atomicAdd(&n_parallel, 1);
-          if (at < kMaxParallel) {
-            parallel[at] = ray;
-            continue;
+#pragma unroll 1
+      for (int shared = 0; shared < 2; shared++) {
+        const int count = shared ? min(n_parallel, kMaxParallel) : nrays;
+#pragma unroll 1
+        for (int i = shared ? 0 : tid; i < count; i += shared ? 1 : T) {
+          float r[6];
+          ray_ends(shared ? parallel[i] : i, r);
+          if (!shared && (r[0] == r[3] || r[1] == r[4] || r[2] == r[5])) {
+            const int at = atomicAdd(&n_parallel, 1);
+            if (at < kMaxParallel) {
+              parallel[at] = i;
+              continue;
+            }
           }
+          walk_ray<OISO>(g, ch, r, shared ? 0 : part, emit, kix, &bad_walk, shared ? tid : 0, shared ? T : 1);
         }
-        walk_ray<OISO>(g, ch, r, part, emit, kix, &bad_walk, 0, 1);
-      }
-      __syncthreads();
-      const int np = min(n_parallel, kMaxParallel);
-      for (int i = 0; i < np; i++) {
-        float r[6];
-        ray_ends(parallel[i], r);
-        walk_ray<OISO>(g, ch, r, 0, emit, kix, &bad_walk, tid, T);
+        __syncthreads();
       }
     }
-    __syncthreads();
     if (overflow || bad_walk) {
       if (tid == 0) {
         row_nnz[bi] = -1;
