@@ -1308,7 +1308,8 @@ __global__ void __launch_bounds__(T, rest_blocks(H))
       }
     };
     const int cnl = cnl_ids[row0 + bi];  // in range: the slab kernel has looked
-    __syncthreads();                     // the previous row's use of the shared memory is over
+    // (see sm_table_kernel)
+    if (__syncthreads_or(tid == 0 && (*(volatile int32_t*)flags & 1) != 0)) break;
     if (tid == 0) {
       channel_setup(g, sincos, cnl, ch);
       bad_walk = to_table = outside = win_u = win_v = 0;
@@ -1340,10 +1341,7 @@ __global__ void __launch_bounds__(T, rest_blocks(H))
     }
     __syncthreads();
     const int wu = win_u, wv = win_v, W = wu * wv;
-    if ((long long)na * wu * wv >= (long long)window_floats(H)) {
-      table(1);
-      continue;
-    }
+    if ((long long)na * wu * wv >= (long long)window_floats(H)) continue;  // for the table kernel, which counts it
     const int nslots = na * W;
     for (int sl = tid; sl < na; sl += T) {
       auto at = [&](int k) { return k * W - ulo[k] * wv - vlo[k]; };
@@ -1503,7 +1501,9 @@ __global__ void __launch_bounds__(T, rest_blocks(H)) sm_table_kernel(DGeom g, co
       }
       continue;
     }
-    __syncthreads();  // the previous row's use of the shared memory is over
+    // the previous row's use of the shared memory is over; once a row has
+    // overflowed, its whole chunk is built again a level up
+    if (__syncthreads_or(tid == 0 && (*(volatile int32_t*)flags & 1) != 0)) break;
     if (tid == 0) {
       channel_setup(g, sincos, cnl, ch);
       overflow = 0;
