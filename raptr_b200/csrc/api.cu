@@ -960,7 +960,7 @@ raptr_status transpose_impl(int64_t m, int64_t n, const int64_t* d_row_ptr, cons
       part(w.off, tasks + 1);
       part(w.scan_tmp, scan_temp_elems(std::max(nh, tasks)));
       part(w.tile_first, sorted.bins + 1);
-      part(w.flags, 1);
+      part(w.flags, 2);
       part(w.split, int64_t(sorted.bins + 1) * m);
     };
     auto lay_staging = [&](char* p) {
@@ -972,19 +972,19 @@ raptr_status transpose_impl(int64_t m, int64_t n, const int64_t* d_row_ptr, cons
       part(w.st_v, nnz);
       part(w.st_low, nnz);
     };
-    int32_t h_flags = -1;  // the ways below may need less memory
+    int32_t h_flags[2] = {-1, 0};  // the ways below may need less memory
     cudaError_t e = cudaSuccess;
     lay_small(nullptr);
     if (dev_malloc(&small, bytes) == cudaSuccess) {
       lay_small(small);
       e = launch_sorted_split(sorted, m, n, nnz, d_row_ptr, d_col, d_order, w, s);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(&h_flags, w.flags, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(h_flags, w.flags, sizeof(h_flags), cudaMemcpyDeviceToHost, s);
       const cudaError_t e2 = cudaStreamSynchronize(s);
       if (e == cudaSuccess) e = e2;
       lay_staging(nullptr);
-      if (e == cudaSuccess && h_flags == 0 && dev_malloc(&staging, bytes) == cudaSuccess) {
+      if (e == cudaSuccess && h_flags[0] == 0 && dev_malloc(&staging, bytes) == cudaSuccess) {
         lay_staging(staging);
-        e = launch_sorted_move(sorted, m, n, nnz, d_col, d_val, w, d_col_ptr, d_row_idx, d_tval, s);
+        e = launch_sorted_move(sorted, m, n, nnz, h_flags[1], d_col, d_val, w, d_col_ptr, d_row_idx, d_tval, s);
         const cudaError_t e3 = cudaStreamSynchronize(s);
         if (e == cudaSuccess) e = e3;
       }
@@ -993,9 +993,9 @@ raptr_status transpose_impl(int64_t m, int64_t n, const int64_t* d_row_ptr, cons
     if (e == cudaSuccess && !done) (void)cudaGetLastError();
     dev_free(staging);
     dev_free(small);
-    if (trace_on()) trace("transpose of sorted rows: %.2f ms, flags %d", trace_ms() - t0, int(h_flags));
+    if (trace_on()) trace("transpose of sorted rows: %.2f ms, flags %d", trace_ms() - t0, int(h_flags[0]));
     if (e != cudaSuccess) return cuda_fail(e, "raptr_csr_transpose");
-    if (h_flags > 0 && (h_flags & 1)) return fail(RAPTR_ERR_INVALID, "column index or row order entry out of range");
+    if (h_flags[0] > 0 && (h_flags[0] & 1)) return fail(RAPTR_ERR_INVALID, "column index or row order entry out of range");
     if (done) return RAPTR_OK;
   }
   // Otherwise: radix sort by column when it applies and its staging (12 bytes per

@@ -293,7 +293,7 @@ struct SortedScratch {
   int64_t* off = nullptr;         // bins * blocks + 1
   int64_t* scan_tmp = nullptr;    // scan_temp_elems of bins * blocks or sorted_hist_elems, the larger
   int32_t* tile_first = nullptr;  // bins + 1
-  int32_t* flags = nullptr;       // 1
+  int32_t* flags = nullptr;       // 2: the flags, and the entries of the largest piece if they are many (`most`)
   uint16_t* split = nullptr;      // (bins + 1) * m
   // the first
   int64_t* size = nullptr;        // bins * blocks
@@ -308,7 +308,7 @@ bool transpose_sorted_plan(int64_t m, int64_t n, int64_t nnz, SortedPlan* p);
 int64_t sorted_hist_elems(const SortedPlan& p);
 cudaError_t launch_sorted_split(const SortedPlan& p, int64_t m, int64_t n, int64_t nnz, const int64_t* rp,
                                 const int32_t* col, const int32_t* order, const SortedScratch& w, cudaStream_t s);
-cudaError_t launch_sorted_move(const SortedPlan& p, int64_t m, int64_t n, int64_t nnz, const int32_t* col,
+cudaError_t launch_sorted_move(const SortedPlan& p, int64_t m, int64_t n, int64_t nnz, int most, const int32_t* col,
                                const float* val, const SortedScratch& w, int64_t* cp, int32_t* trow, float* tval,
                                cudaStream_t s);
 
