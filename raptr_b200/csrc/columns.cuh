@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -29,51 +30,41 @@ __device__ __forceinline__ void two_sum_add(float& s, float& c, float v) {
   s = t;
 }
 
-// A sum in FP32: plain, or with its compensation (the FP16 form's).
-struct PlainSum {
-  float s = 0.f;
-  __device__ __forceinline__ void add(float v) { s += v; }
-  __device__ __forceinline__ void add(const PlainSum& o) { s += o.s; }
-  __device__ __forceinline__ PlainSum from_lane_xor(int o) const {
-    PlainSum r;
-    r.s = __shfl_xor_sync(0xffffffffu, s, o);
-    return r;
-  }
-  __device__ __forceinline__ float value() const { return s; }
-};
+// An FP32 sum with its compensation.
 struct CompensatedSum {
   float s = 0.f, c = 0.f;
-  __device__ __forceinline__ void add(float v) { two_sum_add(s, c, v); }
-  __device__ __forceinline__ void add(const CompensatedSum& o) {
-    two_sum_add(s, c, o.s);
-    c += o.c;
+  __device__ __forceinline__ void add_lane_xor(const CompensatedSum& o, int x) {
+    const float so = __shfl_xor_sync(0xffffffffu, o.s, x), co = __shfl_xor_sync(0xffffffffu, o.c, x);
+    two_sum_add(s, c, so);
+    c += co;
   }
-  __device__ __forceinline__ CompensatedSum from_lane_xor(int o) const {
-    CompensatedSum r;
-    r.s = __shfl_xor_sync(0xffffffffu, s, o);
-    r.c = __shfl_xor_sync(0xffffffffu, c, o);
-    return r;
-  }
-  __device__ __forceinline__ float value() const { return s + c; }
 };
 
 // Sums of four values over the warp: lane l gets that of value l / 8.
-template <class Sum>
-__device__ __forceinline__ float warp_sum4(const Sum (&s)[4], int lane) {
+__device__ __forceinline__ float warp_sum4(const float (&s)[4], int lane) {
   const bool h = (lane & 16) != 0, q = (lane & 8) != 0;
-  Sum a = h ? s[2] : s[0], b = h ? s[3] : s[1];
-  a.add((h ? s[0] : s[2]).from_lane_xor(16));
-  b.add((h ? s[1] : s[3]).from_lane_xor(16));
-  Sum t = q ? b : a;
-  t.add((q ? a : b).from_lane_xor(8));
+  float a = (h ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, h ? s[0] : s[2], 16);
+  float b = (h ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, h ? s[1] : s[3], 16);
+  a = (q ? b : a) + __shfl_xor_sync(0xffffffffu, q ? a : b, 8);
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) t.add(t.from_lane_xor(o));
-  return t.value();
+  for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  return a;
+}
+__device__ __forceinline__ float warp_sum4(const CompensatedSum (&s)[4], int lane) {
+  const bool h = (lane & 16) != 0, q = (lane & 8) != 0;
+  CompensatedSum a = h ? s[2] : s[0], b = h ? s[3] : s[1];
+  a.add_lane_xor(h ? s[0] : s[2], 16);
+  b.add_lane_xor(h ? s[1] : s[3], 16);
+  CompensatedSum t = q ? b : a;
+  t.add_lane_xor(q ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) t.add_lane_xor(t, o);
+  return t.s + t.c;
 }
 
-// Dot products of four columns of at most kShortColumn entries with e, in
-// sums of type Sum; lane l gets that of column l / 8.  All loads of the four are
-// in flight together.
+// Dot products of four columns of at most kShortColumn entries with e, in sums
+// of type Sum (float, or CompensatedSum: the FP16 form); lane l gets that of column
+// l / 8.  All loads of the four are in flight together.
 template <class Sum, class VT, class F>
 __device__ __forceinline__ float short_columns(const int32_t* __restrict__ trow, const VT* __restrict__ tval,
                                                const int64_t (&b)[4], const int (&len)[4],
@@ -91,9 +82,16 @@ __device__ __forceinline__ float short_columns(const int32_t* __restrict__ trow,
     }
 #pragma unroll
   for (int k = 0; k < 4; k++) {
+    if constexpr (std::is_same_v<Sum, float>) {
+      s[k] = 0.f;
 #pragma unroll
-    for (int u = 0; u < 2; u++)
-      if (r[k][u] >= 0) s[k].add(to_float(w[k][u]) * __ldg(e + r[k][u]));
+      for (int u = 0; u < 2; u++)
+        if (r[k][u] >= 0) s[k] += to_float(w[k][u]) * __ldg(e + r[k][u]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 2; u++)
+        if (r[k][u] >= 0) two_sum_add(s[k].s, s[k].c, to_float(w[k][u]) * __ldg(e + r[k][u]));
+    }
   }
   return warp_sum4(s, lane);
 }

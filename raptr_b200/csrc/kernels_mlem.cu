@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(kThreads, kBackBlocks) mlem_back_kernel(int64_
   const double sum = back_columns<UPDATE>(
       n, cp, x, sens, out, next, [&](int64_t b, int64_t b1) { return col_dot<VEC>(trow, tval, b, b1, e, lane); },
       [&](const int64_t(&b)[4], const int(&len)[4]) {
-        return short_columns<PlainSum>(trow, tval, b, len, e, lane, [](float v) { return v; });
+        return short_columns<float>(trow, tval, b, len, e, lane, [](float v) { return v; });
       });
   if (UPDATE) block_add_double(sum, acc);
 }
