@@ -13,6 +13,12 @@ constexpr int kShortColumn = 64;    // entries of a column that four are taken o
 
 constexpr int kColumnCost = 64;     // entries that the looking at a column counts for
 
+// Columns up to which the back pass has a warp for each (EACH below).  In units, few
+// columns fall to few warps, and the draws are as many as without units: FP32 back
+// projection of 300 columns of 5,000 entries 41 us in units, 23 so; 50 of 40 20 and 11;
+// 18,000 of 1,000 77 and 75.
+constexpr int64_t kEachColumn = 148 * 16 * 8;
+
 // Count of a unit of columns, of `total` in all: 32 units to a warp that is
 // resident, but no less than a draw takes to serve (2048 entries).
 __device__ __forceinline__ int64_t column_unit(int64_t total) {
@@ -116,19 +122,25 @@ __device__ __forceinline__ float short_columns(const int32_t* __restrict__ trow,
 // 31 / 31 us, 20,000 rows 252 / 248 -> 54 / 52, 200,000 rows 528 / 460 -> 224 /
 // 193, 5.14M rows (100 rays) 4.3 / 3.4 -> 4.1 / 3.5 ms; units of 1024 or 4096
 // entries and 8 or 16 units to a warp are 2-10 % slower on some of these.
-template <bool UPDATE, class Dot, class Dot4>
+//
+// With EACH, for few columns, there are no units: every warp takes a column, and
+// neighbours (which may be long together) go to different blocks.
+template <bool UPDATE, bool EACH, class Dot, class Dot4>
 __device__ __forceinline__ double back_columns(int64_t n, const int64_t* __restrict__ cp,
                                                const float* __restrict__ x, const float* __restrict__ sens,
                                                float* __restrict__ out, unsigned long long* next, Dot dot,
                                                Dot4 dot4) {
   const int lane = threadIdx.x & 31;
-  const int64_t total = cp[n] + kColumnCost * n, unit = column_unit(total);
+  const int64_t total = EACH ? n : cp[n] + kColumnCost * n, unit = EACH ? 1 : column_unit(total);
+  if (EACH) next = nullptr;
   double sum = 0.0;
-  int64_t k = next ? warp_next(next, lane) : (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  int64_t k = EACH   ? int64_t(threadIdx.x >> 5) * gridDim.x + blockIdx.x
+              : next ? warp_next(next, lane)
+                     : (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   while (k * unit < total) {
     const int64_t p0 = k * unit, p1 = p0 + unit;
     // the first column at p0 or later, 32 probes at a time
-    int64_t j0 = 0, hi = n;
+    int64_t j0 = EACH ? k : 0, hi = EACH ? k : n;
     while (j0 < hi) {
       const int64_t step = (hi - j0 + 31) >> 5, j = j0 + lane * step;
       const bool before = j < hi && cp[j] + kColumnCost * j < p0;
@@ -145,7 +157,7 @@ __device__ __forceinline__ double back_columns(int64_t n, const int64_t* __restr
       if (j < n) {
         b = cp[j];
         e = cp[j + 1];
-        own = b + kColumnCost * j < p1;
+        own = EACH ? j == k : b + kColumnCost * j < p1;
       }
       more = __all_sync(0xffffffffu, own);
       const int len = own ? int(min(e - b, int64_t(kShortColumn + 1))) : 0;

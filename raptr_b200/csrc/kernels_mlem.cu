@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(kThreads, kPassBlocks) mlem_forward_kernel(int
 // (`next`, zero at launch) the warps draw columns from it (back_columns): a
 // grid stride leaves the kernel waiting on the warps that drew the longest
 // (0.85 instead of 0.72 of HBM on the 70^3 x 5.14M matrix).
-template <bool VEC, bool UPDATE>
+template <bool VEC, bool UPDATE, bool EACH>
 __global__ void __launch_bounds__(kThreads, kBackBlocks) mlem_back_kernel(int64_t n, const int64_t* __restrict__ cp,
                                                              const int32_t* __restrict__ trow,
                                                              const float* __restrict__ tval,
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(kThreads, kBackBlocks) mlem_back_kernel(int64_
                                                              const float* __restrict__ sens, float* __restrict__ out,
                                                              double* __restrict__ acc, unsigned long long* next) {
   const int lane = threadIdx.x & 31;
-  const double sum = back_columns<UPDATE>(
+  const double sum = back_columns<UPDATE, EACH>(
       n, cp, x, sens, out, next, [&](int64_t b, int64_t b1) { return col_dot<VEC>(trow, tval, b, b1, e, lane); },
       [&](const int64_t(&b)[4], const int(&len)[4]) {
         return short_columns<float>(trow, tval, b, len, e, lane, [](float v) { return v; });
@@ -756,25 +756,14 @@ cudaError_t launch_mlem_back(int64_t n, const int64_t* cp, const int32_t* trow, 
                              cudaStream_t s, unsigned long long* next) {
   if (n <= 0) return cudaSuccess;
   const bool v = aligned16(trow, tval);
-  if (update) {
-    if (v) {
-      mlem_back_kernel<true, true><<<row_grid(n), kThreads, 0, s>>>(n, cp, trow, tval, e, x, sens, out, d_acc, next);
-      note_launches(1);
-    }
-    else {
-      mlem_back_kernel<false, true><<<row_grid(n), kThreads, 0, s>>>(n, cp, trow, tval, e, x, sens, out, d_acc, next);
-      note_launches(1);
-    }
-  } else {
-    if (v) {
-      mlem_back_kernel<true, false><<<row_grid(n), kThreads, 0, s>>>(n, cp, trow, tval, e, x, sens, out, d_acc, next);
-      note_launches(1);
-    }
-    else {
-      mlem_back_kernel<false, false><<<row_grid(n), kThreads, 0, s>>>(n, cp, trow, tval, e, x, sens, out, d_acc, next);
-      note_launches(1);
-    }
-  }
+  auto pick = [&](auto each) {
+    constexpr bool E = decltype(each)::value;
+    return update ? (v ? mlem_back_kernel<true, true, E> : mlem_back_kernel<false, true, E>)
+                  : (v ? mlem_back_kernel<true, false, E> : mlem_back_kernel<false, false, E>);
+  };
+  auto kernel = n <= kEachColumn ? pick(std::true_type{}) : pick(std::false_type{});
+  kernel<<<row_grid(n), kThreads, 0, s>>>(n, cp, trow, tval, e, x, sens, out, d_acc, next);
+  note_launches(1);
   return cudaGetLastError();
 }
 

@@ -264,7 +264,7 @@ __device__ __forceinline__ float col_dot_half(const int32_t* __restrict__ trow, 
 }
 
 // Columns as in mlem_back_kernel (back_columns).
-template <bool UPDATE>
+template <bool UPDATE, bool EACH>
 __global__ void __launch_bounds__(kThreads, 4) mlem_back_half_kernel(int64_t n, const int64_t* __restrict__ cp,
                                                                   const int32_t* __restrict__ trow,
                                                                   const uint16_t* __restrict__ htval,
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kThreads, 4) mlem_back_half_kernel(int64_t n, 
                                                                   float* __restrict__ out, double* __restrict__ acc,
                                                                   unsigned long long* next) {
   const int lane = threadIdx.x & 31;
-  const double sum = back_columns<UPDATE>(
+  const double sum = back_columns<UPDATE, EACH>(
       n, cp, x, sens, out, next, [&](int64_t b, int64_t b1) { return col_dot_half(trow, htval, b, b1, e, lane); },
       [&](const int64_t(&b)[4], const int(&len)[4]) {
         return short_columns<CompensatedSum>(trow, reinterpret_cast<const unsigned short*>(htval), b, len, e, lane,
@@ -649,10 +649,10 @@ cudaError_t launch_mlem_back_half(int64_t n, const int64_t* cp, const int32_t* t
                                   const float* e, const float* x, const float* sens, float* out, double* d_acc,
                                   bool update, cudaStream_t s, unsigned long long* next) {
   if (n <= 0) return cudaSuccess;
-  if (update)
-    mlem_back_half_kernel<true><<<grid_rows(n), kThreads, 0, s>>>(n, cp, trow, htval, e, x, sens, out, d_acc, next);
-  else
-    mlem_back_half_kernel<false><<<grid_rows(n), kThreads, 0, s>>>(n, cp, trow, htval, e, x, sens, out, d_acc, next);
+  const bool each = n <= kEachColumn;
+  auto kernel = update ? (each ? mlem_back_half_kernel<true, true> : mlem_back_half_kernel<true, false>)
+                       : (each ? mlem_back_half_kernel<false, true> : mlem_back_half_kernel<false, false>);
+  kernel<<<grid_rows(n), kThreads, 0, s>>>(n, cp, trow, htval, e, x, sens, out, d_acc, next);
   note_launches(1);
   return cudaGetLastError();
 }
