@@ -165,6 +165,31 @@ __device__ __forceinline__ void row_scatter(const int32_t* __restrict__ col, con
   }
 }
 
+// A row [b, e) of at most 64 entries, the lane's two of it.  The steps of 32 U
+// entries above cost such rows more instructions than they have entries: transposed
+// SpMV of 1M rows of 10 225 us, 175 so; MLEM projection 362 and 272.
+constexpr int kShortRow = 64;
+struct ShortRow {
+  int c0, c1;
+  float v0, v1;
+  __device__ __forceinline__ ShortRow(const int32_t* __restrict__ col, const float* __restrict__ val, int64_t b,
+                                      int64_t e, int lane) {
+    const bool in0 = b + lane < e, in1 = b + lane + 32 < e;
+    c0 = in0 ? __ldcs(col + b + lane) : -1;
+    c1 = in1 ? __ldcs(col + b + lane + 32) : -1;
+    v0 = in0 ? __ldcs(val + b + lane) : 0.f;
+    v1 = in1 ? __ldcs(val + b + lane + 32) : 0.f;
+  }
+  __device__ __forceinline__ float dot(const float* __restrict__ x) const {
+    const float g0 = c0 >= 0 ? __ldg(x + c0) : 0.f, g1 = c1 >= 0 ? __ldg(x + c1) : 0.f;
+    return warp_sum(v0 * g0 + v1 * g1);
+  }
+  __device__ __forceinline__ void scatter(float f, float* __restrict__ y) const {
+    if (c0 >= 0) atomicAdd(y + c0, v0 * f);
+    if (c1 >= 0) atomicAdd(y + c1, v1 * f);
+  }
+};
+
 __global__ void __launch_bounds__(kThreads, kPassBlocks) spmv_n_kernel(int64_t m, const int64_t* __restrict__ rp,
                                                           const int32_t* __restrict__ col,
                                                           const float* __restrict__ val, float alpha,
@@ -186,7 +211,12 @@ __global__ void __launch_bounds__(kThreads) spmv_t_kernel(int64_t m, const int64
   const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
   for (int64_t r = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; r < m; r += nw) {
     float f = alpha * x[r];
-    if (f != 0.f) row_scatter<8>(col, val, rp[r], rp[r + 1], f, y, lane);
+    if (f == 0.f) continue;
+    const int64_t b = rp[r], e = rp[r + 1];
+    if (e - b <= kShortRow)
+      ShortRow(col, val, b, e, lane).scatter(f, y);
+    else
+      row_scatter<8>(col, val, b, e, f, y, lane);
   }
 }
 
@@ -277,6 +307,18 @@ __global__ void __launch_bounds__(kNormThreads) sens_norm_self_kernel(int64_t n,
   for (int64_t i = threadIdx.x; i < n; i += kNormThreads) s32[i] = float(s64[i] / t);
 }
 
+// The projection of a short row; returns its dot product.  A function of its own,
+// so that the long rows' loops keep their registers (inlined, 10 rows of 60,000 take 359 us
+// instead of 338).
+__device__ __noinline__ float short_project(const int32_t* __restrict__ col, const float* __restrict__ val, int64_t b,
+                                            int64_t e, float yi, const float* __restrict__ x, float* __restrict__ c,
+                                            int lane) {
+  const ShortRow row(col, val, b, e, lane);
+  const float yt = row.dot(x);
+  row.scatter(__fdiv_rn(yi, yt), c);
+  return yt;
+}
+
 // Fused MLEM projection: per measured row, yt = <a_i, x>, e = y_i / yt
 // (no zero guard, src/mlemOperations.hpp:44-54), c += e * a_i.  A row with
 // y_i == 0 is not part of the measurement (the reference's matrix has no row
@@ -294,13 +336,14 @@ __global__ void __launch_bounds__(kThreads) mlem_project_kernel(int64_t m, const
     const float yi = __ldg(y + r);
     if (yi == 0.f) continue;
     const int64_t b = rp[r], e = rp[r + 1];
-    const float yt = row_dot_seq<8>(col, val, b, e, x, lane);
+    const bool is_short = e - b <= kShortRow;
+    const float yt = is_short ? short_project(col, val, b, e, yi, x, c, lane) : row_dot_seq<8>(col, val, b, e, x, lane);
     const float f = __fdiv_rn(yi, yt);
     if (ll && lane == 0) {
       ly += double(yi) * log(double(yt));
       lt += double(yt);
     }
-    row_scatter<8>(col, val, b, e, f, c, lane);
+    if (!is_short) row_scatter<8>(col, val, b, e, f, c, lane);
   }
   if (ll) {
     block_add_double(ly, ll);
