@@ -283,10 +283,11 @@ __device__ __forceinline__ int64_t warp_next(unsigned long long* next, int lane)
   return int64_t(__shfl_sync(0xffffffffu, q, 0));
 }
 
-// Below this many rows (eight to a warp) the row passes take them by a grid
-// stride, since the draws would take longer than the rows (28,561 rows of 438
-// entries: 47 us drawn, 31 us strided; 57,122 of 1535: 157 drawn, 164 strided).
-constexpr int64_t kDrawRows = int64_t(kDrawWarps) * 8;
+// Below this many rows, each of which would be a draw of its own, the row passes take
+// them by a grid stride, since the draws would take longer than the rows: 57,122 rows
+// of 438 entries 73 us drawn, 51 strided; 94,000 of 724 131 and 117.  (Rows of 1535
+// entries are 1-2 % faster drawn: 57,122 155 and 158.)
+constexpr int64_t kDrawRows = int64_t(kDrawWarps) * 16;
 
 // Rows a draw takes: 16 (one draw per row makes the forward pass of 5.14M rows
 // twice as slow, one per 16 takes 7 % off the grid stride's time), fewer where
