@@ -126,7 +126,23 @@ __global__ void __launch_bounds__(kThreads, kForwardBlocks) batch_forward_kernel
     float acc[S::VEC];
 #pragma unroll
     for (int v = 0; v < S::VEC; v++) acc[v] = 0.f;
-    gather_entries<KT>(col, val, rp[r], rp[r + 1], X, xs, lane, acc);
+    const int64_t b = rp[r], e = rp[r + 1];
+    if constexpr (KT == 8) {
+      // (as gather_entries, whose loop is compiled differently here: 5.14M rows of 70^3,
+      // FP16, 11.2 ms, so 10.2; every other width is as fast or faster with it)
+      int64_t k = b + es;
+      for (; k + S::EPW < e; k += 2 * S::EPW) {
+        const int c0 = __ldg(col + k), c1 = __ldg(col + k + S::EPW);
+        const float w0 = to_f(val[k]), w1 = to_f(val[k + S::EPW]);
+        const float4 x0 = ld4(X + int64_t(c0) * xs);
+        const float4 x1 = ld4(X + int64_t(c1) * xs);
+        fma4(acc, w0, x0);
+        fma4(acc, w1, x1);
+      }
+      if (k < e) fma4(acc, to_f(val[k]), ld4(X + int64_t(__ldg(col + k)) * xs));
+    } else {
+      gather_entries<KT>(col, val, b, e, X, xs, lane, acc);
+    }
 #pragma unroll
     for (int o = S::LPE; o < 32; o <<= 1)
 #pragma unroll
