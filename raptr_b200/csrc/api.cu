@@ -1714,7 +1714,8 @@ raptr_status raptr_sensitivity_half(int64_t n, const int64_t* d_col_ptr, const i
 
 // ---- batched MLEM ----------------------------------------------------------
 
-namespace {
+extern "C++" {
+namespace raptr {
 
 raptr_status batch_args(raptr_ctx* ctx, int64_t m, int64_t n, int32_t K, int32_t value_type, const int64_t* d_row_ptr,
                         const int32_t* d_col, const void* d_val, const float* d_rscale, const int64_t* d_col_ptr,
@@ -1745,50 +1746,68 @@ raptr_status batch_args(raptr_ctx* ctx, int64_t m, int64_t n, int32_t K, int32_t
   return RAPTR_OK;
 }
 
+namespace {
+
 // The widest tile: 64 frames of 70^3 x 5.14M channels take 105 ms an iteration in
 // one tile of 64 and 112 in two of 32, of x 57,122 channels 1.53 and 1.92.
 int default_frame_tile(int K) { return batch_tile_supported(K, 64) ? 64 : 0; }
 
+// The list of columns into cols, their number into *n_full, one of the n + (n + 1) +
+// scan_temp_elems(n) 64-bit words taken from cv.  The tube order of the back pass
+// applies when the columns are the context's voxels.
+raptr_status list_columns(raptr_ctx* ctx, int64_t n, const int64_t* d_col_ptr, Carve& cv, int32_t* cols,
+                          const int64_t** n_full, cudaStream_t s) {
+  const int32_t* order = nullptr;
+  if (n == int64_t(ctx->dg.n[0]) * ctx->dg.n[1] * ctx->dg.n[2]) RCU(ctx->col_order(s, &order));
+  int64_t* flag = cv.take<int64_t>(size_t(n));
+  int64_t* pos = cv.take<int64_t>(size_t(n + 1));
+  int64_t* tmp = cv.take<int64_t>(size_t(scan_temp_elems(n)));
+  RCU(launch_batch_columns(n, d_col_ptr, order, flag, pos, tmp, cols, s));
+  *n_full = pos + n;
+  return RAPTR_OK;
+}
+
 }  // namespace
 
-raptr_status raptr_mlem_batch(raptr_ctx* ctx, int64_t m, int64_t n, int32_t n_frames, int32_t value_type,
-                              const int64_t* d_row_ptr, const int32_t* d_col, const void* d_val,
-                              const float* d_rscale, const int64_t* d_col_ptr, const int32_t* d_row_idx,
-                              const void* d_tval, const int32_t* d_row_rank, const float* d_y, const float* d_s,
-                              float* d_x, int32_t n_iter, int32_t frame_tile, const raptr_mlem_opts* opts,
-                              void* stream) {
-  BatchArgs a;
-  RCHECK(batch_args(ctx, m, n, n_frames, value_type, d_row_ptr, d_col, d_val, d_rscale, d_col_ptr, d_row_idx, d_tval,
-                    d_row_rank, d_y, d_s, d_x, &a));
+raptr_status batch_columns(raptr_ctx* ctx, int64_t n, const int64_t* d_col_ptr, int32_t* cols, int64_t* n_full,
+                           cudaStream_t s) {
+  DeviceScope ds(ctx->device);
+  RCHECK(ctx->ensure_scratch(Carve::need({size_t(n) * sizeof(int64_t), size_t(n + 1) * sizeof(int64_t),
+                                          size_t(scan_temp_elems(n)) * sizeof(int64_t)})));
+  Carve cv(ctx->d_scratch);
+  const int64_t* count = nullptr;
+  RCHECK(list_columns(ctx, n, d_col_ptr, cv, cols, &count, s));
+  RCU(cudaMemcpyAsync(n_full, count, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
+  return RAPTR_OK;
+}
+
+raptr_status mlem_batch(raptr_ctx* ctx, BatchArgs a, int32_t n_iter, int32_t frame_tile, const raptr_mlem_opts* opts,
+                        cudaStream_t s) {
+  const int64_t m = a.m, n = a.n;
+  const int32_t n_frames = a.K;
   if (n_iter < 0) return fail(RAPTR_ERR_INVALID, "bad argument");
   const int kt = frame_tile > 0 ? frame_tile : default_frame_tile(n_frames);
   if (!batch_tile_supported(n_frames, kt))
     return fail(RAPTR_ERR_INVALID, "the number of frames must be a multiple of 4 and the frame tile 4, 8, 16, 32 or 64");
   if (n_iter == 0) return RAPTR_OK;
   DeviceScope ds(ctx->device);
-  cudaStream_t s = as_stream(stream);
   const bool want_times = opts && opts->h_kernel_ms;
   const bool wait = opts && opts->use_graph && !want_times;
+  const bool listed = a.cols != nullptr;
   RCHECK(ctx->ensure_scratch(Carve::need({size_t(std::max<int64_t>(m, 1)) * n_frames * sizeof(float),
                                           size_t(n) * n_frames * sizeof(float), size_t(n_frames) * sizeof(double),
                                           size_t(n_frames) * sizeof(unsigned long long) * kBatchRowBlocks,
-                                          size_t(n) * sizeof(int64_t), size_t(n + 1) * sizeof(int64_t),
-                                          size_t(scan_temp_elems(n)) * sizeof(int64_t), size_t(n) * sizeof(int32_t),
+                                          listed ? 0 : size_t(n) * sizeof(int64_t),
+                                          listed ? 0 : size_t(n + 1) * sizeof(int64_t),
+                                          listed ? 0 : size_t(scan_temp_elems(n)) * sizeof(int64_t),
+                                          listed ? 0 : size_t(n) * sizeof(int32_t),
                                           size_t(n) * std::min(kt, int(n_frames)) * sizeof(float),
                                           size_t(n) * batch_tile_at(n_frames, kt, 0) * sizeof(float)})));
   Carve cv(ctx->d_scratch);
-  // the tube order of the back pass applies when the columns are the
-  // context's voxels
-  const int32_t* order = nullptr;
-  if (n == int64_t(ctx->dg.n[0]) * ctx->dg.n[1] * ctx->dg.n[2]) RCU(ctx->col_order(s, &order));
-  {
-    int64_t* flag = cv.take<int64_t>(size_t(n));
-    int64_t* pos = cv.take<int64_t>(size_t(n + 1));
-    int64_t* tmp = cv.take<int64_t>(size_t(scan_temp_elems(n)));
+  if (!a.cols) {
     int32_t* cols = cv.take<int32_t>(size_t(n));
-    RCU(launch_batch_columns(n, d_col_ptr, order, flag, pos, tmp, cols, s));
+    RCHECK(list_columns(ctx, n, a.cp, cv, cols, &a.n_full, s));
     a.cols = cols;
-    a.n_full = pos + n;
   }
   a.E = cv.take<float>(size_t(std::max<int64_t>(m, 1)) * n_frames);
   a.XX = cv.take<float>(size_t(n) * n_frames);
@@ -1800,7 +1819,7 @@ raptr_status raptr_mlem_batch(raptr_ctx* ctx, int64_t m, int64_t n, int32_t n_fr
   if (widest < n_frames) a.Xt = cv.take<float>(size_t(n) * widest);
   // the back pass in row-block groups when one tile's ratios exceed L2
   if (m > 0 && double(m) * std::min(kt, int(n_frames)) * sizeof(float) > kBatchBlockingBytes) {
-    RCU(ctx->block_seg(d_col_ptr, d_row_idx, m, n, s, &a.seg));
+    RCU(ctx->block_seg(a.cp, a.trow, m, n, s, &a.seg));
     a.seg_blocks = kBatchRowBlocks;
     a.P = cv.take<float>(size_t(n) * std::min(kt, int(n_frames)));
   }
@@ -1833,6 +1852,21 @@ raptr_status raptr_mlem_batch(raptr_ctx* ctx, int64_t m, int64_t n, int32_t n_fr
     for (auto& ev : evs) cudaEventDestroy(ev);
   }
   return RAPTR_OK;
+}
+
+}  // namespace raptr
+}
+
+raptr_status raptr_mlem_batch(raptr_ctx* ctx, int64_t m, int64_t n, int32_t n_frames, int32_t value_type,
+                              const int64_t* d_row_ptr, const int32_t* d_col, const void* d_val,
+                              const float* d_rscale, const int64_t* d_col_ptr, const int32_t* d_row_idx,
+                              const void* d_tval, const int32_t* d_row_rank, const float* d_y, const float* d_s,
+                              float* d_x, int32_t n_iter, int32_t frame_tile, const raptr_mlem_opts* opts,
+                              void* stream) {
+  BatchArgs a;
+  RCHECK(batch_args(ctx, m, n, n_frames, value_type, d_row_ptr, d_col, d_val, d_rscale, d_col_ptr, d_row_idx, d_tval,
+                    d_row_rank, d_y, d_s, d_x, &a));
+  return mlem_batch(ctx, a, n_iter, frame_tile, opts, as_stream(stream));
 }
 
 raptr_status raptr_mlem_batch_autotune(raptr_ctx* ctx, int64_t m, int64_t n, int32_t n_frames, int32_t value_type,

@@ -237,6 +237,17 @@ cudaError_t launch_block_seg(int64_t n, int64_t m, int B, const int64_t* cp, con
 // as they are); flag n, pos n + 1 (pos + n is n_full), scan_tmp scan_temp_elems(n).
 cudaError_t launch_batch_columns(int64_t n, const int64_t* cp, const int32_t* order, int64_t* flag, int64_t* pos,
                                  int64_t* scan_tmp, int32_t* cols, cudaStream_t s);
+// raptr_mlem_batch in two parts, for callers that iterate one matrix again and
+// again: its list of columns (cols n, n_full one; made with the context's scratch), and
+// the iterations with it.
+raptr_status batch_columns(raptr_ctx* ctx, int64_t n, const int64_t* d_col_ptr, int32_t* cols, int64_t* n_full,
+                           cudaStream_t s);
+raptr_status mlem_batch(raptr_ctx* ctx, BatchArgs a, int32_t n_iter, int32_t frame_tile, const raptr_mlem_opts* opts,
+                        cudaStream_t s);
+raptr_status batch_args(raptr_ctx* ctx, int64_t m, int64_t n, int32_t K, int32_t value_type, const int64_t* d_row_ptr,
+                        const int32_t* d_col, const void* d_val, const float* d_rscale, const int64_t* d_col_ptr,
+                        const int32_t* d_row_idx, const void* d_tval, const int32_t* d_row_rank, const float* d_y,
+                        const float* d_s, float* d_x, BatchArgs* a);
 // K frames (a multiple of 4) in tiles of at most kt (4, 8, 16, 32 or 64).
 bool batch_tile_supported(int K, int kt);
 // The tile that starts at frame f0: kt while kt frames remain, else the

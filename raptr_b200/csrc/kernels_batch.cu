@@ -164,7 +164,9 @@ __global__ void __launch_bounds__(kThreads, kForwardBlocks) batch_forward_kernel
 // ratios; FP32, the FP16 values dominate its error),
 // XX = X*c/(S+(S==0)), acc[f] += sum_j XX (FP64).  Warps take the columns that
 // have entries (the first *n_full of cols) from the counter *next (zero at
-// launch); the others are batch_empty_kernel's.
+// launch).  The others (where few views are measured two thirds of them) have c =
+// 0, so XX = X*0/(S+(S==0)), which is 0 unless X is not finite; the threads of the last
+// group's pass share them afterwards.
 //
 // With a row-block group (seg non-null), only the column's entries whose
 // rows lie in blocks [b0, b1) of the transpose's row order are summed
@@ -252,27 +254,20 @@ __global__ void __launch_bounds__(kThreads, kBackBlocks) batch_back_kernel(int64
   __syncthreads();
   for (int i = threadIdx.x; i < KT; i += blockDim.x)
     if (red[i] != 0.0) atomicAdd(acc + f0 + i, red[i]);
-}
-
-// The update of the columns without entries (cols[*n_full] on, where few views
-// are measured two thirds of them): c = 0, so XX = X*0/(S+(S==0)), which is 0
-// unless X is not finite; acc gets it then.
-__global__ void __launch_bounds__(kThreads) batch_empty_kernel(int64_t n, int K, const int32_t* __restrict__ cols,
-                                                               const int64_t* __restrict__ n_full,
-                                                               const float* __restrict__ X,
-                                                               const float* __restrict__ sens,
-                                                               float* __restrict__ XX, double* __restrict__ acc) {
-  const int64_t first = *n_full;
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < (n - first) * K;
-       i += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t q = i / K;
-    const int f = int(i - q * K);
-    const int64_t j = __ldg(cols + first + q);
-    float dvs = __ldg(sens + j);
-    dvs += float(dvs == 0.f);
-    const float xx = __fdiv_rn(__fmul_rn(X[j * K + f], 0.f), dvs);
-    XX[j * K + f] = xx;
-    if (xx != 0.f) atomicAdd(acc + f, double(xx));
+  if (mode == 0 || mode == 3) {
+    const int64_t empty = (n - int64_t(count)) * S::LPE;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < empty; i += int64_t(gridDim.x) * blockDim.x) {
+      const int64_t j = __ldg(cols + int64_t(count) + i / S::LPE);
+      const int f = f0 + int(i % S::LPE) * S::VEC;
+      float dvs = __ldg(sens + j);
+      dvs += float(dvs == 0.f);
+#pragma unroll
+      for (int v = 0; v < S::VEC; v++) {
+        const float xx = __fdiv_rn(__fmul_rn(X[j * K + f + v], 0.f), dvs);
+        XX[j * K + f + v] = xx;
+        if (xx != 0.f) atomicAdd(acc + f + v, double(xx));
+      }
+    }
   }
 }
 
@@ -474,8 +469,6 @@ cudaError_t launch_batch_iteration(const BatchArgs& a, int kt, double* acc, unsi
     }
   }
   if (e == cudaSuccess) {
-    batch_empty_kernel<<<148 * 8, kThreads, 0, s>>>(a.n, a.K, a.cols, a.n_full, a.X, a.S, a.XX, acc);
-    note_launches(1);
     const int64_t q = a.K / 4;
     const int64_t threads = std::min<int64_t>(a.n * q, std::max<int64_t>(int64_t(148) * 8 * kThreads / q, 1) * q);
     batch_normalise_kernel<<<unsigned((threads + kThreads - 1) / kThreads), kThreads, 0, s>>>(a.n, a.K, threads, a.X,

@@ -137,6 +137,10 @@ struct Entry {
   uint16_t* htval = nullptr;
   int32_t* rank = nullptr;
   float* s = nullptr;
+  // the back pass's columns, listed once (an iteration at a time would list them
+  // anew in each, and every kernel more waits for its turn among the other batches')
+  int32_t* cols = nullptr;
+  int64_t* n_full = nullptr;
   cudaStream_t stream = nullptr;
   std::vector<Request*> active;
   bool dirty = true;
@@ -258,12 +262,15 @@ raptr_status raptr_server::build(Entry* e, std::string* err) {
   double* s64 = nullptr;
   ce = cudaMalloc(&s64, size_t(e->n) * sizeof(double));
   if (ce == cudaSuccess) ce = cudaMalloc(&e->s, size_t(e->n) * sizeof(float));
+  if (ce == cudaSuccess) ce = cudaMalloc(&e->cols, size_t(e->n) * sizeof(int32_t));
+  if (ce == cudaSuccess) ce = cudaMalloc(&e->n_full, sizeof(int64_t));
   if (ce != cudaSuccess) {
     cudaFree(s64);
     *err = cudaGetErrorString(ce);
     return RAPTR_ERR_NOMEM;
   }
   st_ = raptr_sensitivity_half(e->n, e->cp, e->trow, e->htval, ps, s64, e->s, e->stream);
+  if (st_ == RAPTR_OK) st_ = batch_columns(e->ctx, e->n, e->cp, e->cols, e->n_full, e->stream);
   cudaStreamSynchronize(e->stream);
   cudaFree(s64);
   if (st_ != RAPTR_OK) {
@@ -271,7 +278,7 @@ raptr_status raptr_server::build(Entry* e, std::string* err) {
     return st_;
   }
   raptr_matrix_bytes(e->A, &e->matrix_bytes);
-  e->matrix_bytes += e->n * int64_t(sizeof(float));
+  e->matrix_bytes += e->n * int64_t(sizeof(float) + sizeof(int32_t));
   this->st.builds++;
   return RAPTR_OK;
 }
@@ -295,6 +302,10 @@ void raptr_server::drop(Entry* e) {
   e->h_ys = nullptr;
   e->kcap = e->K = 0;
   cudaFree(e->s);
+  cudaFree(e->cols);
+  cudaFree(e->n_full);
+  e->cols = nullptr;
+  e->n_full = nullptr;
   if (e->A) raptr_matrix_destroy(e->A);
   if (e->ctx) raptr_ctx_destroy(e->ctx);
   if (e->stream) cudaStreamDestroy(e->stream);
@@ -506,9 +517,12 @@ void raptr_server::loop() {
       } else {
         // all frames in sweeps of at most 64 (a multiple of 4 frames): one
         // 64-frame sweep takes 105 ms at 70^3, two of 32 take 112 ms
-        e->launch_status = raptr_mlem_batch(e->ctx, e->m, e->n, e->K, 1, e->rp, e->col, e->hval, e->rscale, e->cp,
-                                            e->trow, e->htval, e->rank, e->Y, e->s, e->X(), 1, 64, nullptr,
-                                            e->stream);
+        BatchArgs a;
+        e->launch_status = batch_args(e->ctx, e->m, e->n, e->K, 1, e->rp, e->col, e->hval, e->rscale, e->cp, e->trow,
+                                      e->htval, e->rank, e->Y, e->s, e->X(), &a);
+        a.cols = e->cols;
+        a.n_full = e->n_full;
+        if (e->launch_status == RAPTR_OK) e->launch_status = mlem_batch(e->ctx, a, 1, 64, nullptr, e->stream);
         if (e->launch_status != RAPTR_OK) e->launch_error = raptr_last_error();
       }
       cudaEventRecord(e->done_ev, e->stream);
