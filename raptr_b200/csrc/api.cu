@@ -1752,18 +1752,22 @@ namespace {
 // one tile of 64 and 112 in two of 32, of x 57,122 channels 1.53 and 1.92.
 int default_frame_tile(int K) { return batch_tile_supported(K, 64) ? 64 : 0; }
 
-// The list of columns into cols, their number into *n_full, one of the n + (n + 1) +
-// scan_temp_elems(n) 64-bit words taken from cv.  The tube order of the back pass
-// applies when the columns are the context's voxels.
-raptr_status list_columns(raptr_ctx* ctx, int64_t n, const int64_t* d_col_ptr, Carve& cv, int32_t* cols,
-                          const int64_t** n_full, cudaStream_t s) {
+// The list of columns into cols and n_full, by way of list_bytes(n) of scratch.
+// The tube order of the back pass applies when the columns are the context's voxels.
+size_t list_bytes(int64_t n) {
+  return Carve::need({size_t(n) * sizeof(int64_t), size_t(n + 1) * sizeof(int64_t),
+                      size_t(scan_temp_elems(n)) * sizeof(int64_t)});
+}
+raptr_status list_columns(raptr_ctx* ctx, int64_t n, const int64_t* d_col_ptr, unsigned char* scratch, int32_t* cols,
+                          int64_t* n_full, cudaStream_t s) {
+  Carve cv(scratch);
   const int32_t* order = nullptr;
   if (n == int64_t(ctx->dg.n[0]) * ctx->dg.n[1] * ctx->dg.n[2]) RCU(ctx->col_order(s, &order));
   int64_t* flag = cv.take<int64_t>(size_t(n));
   int64_t* pos = cv.take<int64_t>(size_t(n + 1));
   int64_t* tmp = cv.take<int64_t>(size_t(scan_temp_elems(n)));
   RCU(launch_batch_columns(n, d_col_ptr, order, flag, pos, tmp, cols, s));
-  *n_full = pos + n;
+  RCU(cudaMemcpyAsync(n_full, pos + n, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
   return RAPTR_OK;
 }
 
@@ -1772,13 +1776,8 @@ raptr_status list_columns(raptr_ctx* ctx, int64_t n, const int64_t* d_col_ptr, C
 raptr_status batch_columns(raptr_ctx* ctx, int64_t n, const int64_t* d_col_ptr, int32_t* cols, int64_t* n_full,
                            cudaStream_t s) {
   DeviceScope ds(ctx->device);
-  RCHECK(ctx->ensure_scratch(Carve::need({size_t(n) * sizeof(int64_t), size_t(n + 1) * sizeof(int64_t),
-                                          size_t(scan_temp_elems(n)) * sizeof(int64_t)})));
-  Carve cv(ctx->d_scratch);
-  const int64_t* count = nullptr;
-  RCHECK(list_columns(ctx, n, d_col_ptr, cv, cols, &count, s));
-  RCU(cudaMemcpyAsync(n_full, count, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
-  return RAPTR_OK;
+  RCHECK(ctx->ensure_scratch(list_bytes(n)));
+  return list_columns(ctx, n, d_col_ptr, ctx->d_scratch, cols, n_full, s);
 }
 
 raptr_status mlem_batch(raptr_ctx* ctx, BatchArgs a, int32_t n_iter, int32_t frame_tile, const raptr_mlem_opts* opts,
@@ -1786,7 +1785,7 @@ raptr_status mlem_batch(raptr_ctx* ctx, BatchArgs a, int32_t n_iter, int32_t fra
   const int64_t m = a.m, n = a.n;
   const int32_t n_frames = a.K;
   if (n_iter < 0) return fail(RAPTR_ERR_INVALID, "bad argument");
-  const int kt = frame_tile > 0 ? frame_tile : default_frame_tile(n_frames);
+  int kt = frame_tile > 0 ? frame_tile : default_frame_tile(n_frames);
   if (!batch_tile_supported(n_frames, kt))
     return fail(RAPTR_ERR_INVALID, "the number of frames must be a multiple of 4 and the frame tile 4, 8, 16, 32 or 64");
   if (n_iter == 0) return RAPTR_OK;
@@ -1794,34 +1793,51 @@ raptr_status mlem_batch(raptr_ctx* ctx, BatchArgs a, int32_t n_iter, int32_t fra
   const bool want_times = opts && opts->h_kernel_ms;
   const bool wait = opts && opts->use_graph && !want_times;
   const bool listed = a.cols != nullptr;
-  RCHECK(ctx->ensure_scratch(Carve::need({size_t(std::max<int64_t>(m, 1)) * n_frames * sizeof(float),
-                                          size_t(n) * n_frames * sizeof(float), size_t(n_frames) * sizeof(double),
-                                          size_t(n_frames) * sizeof(unsigned long long) * kBatchRowBlocks,
-                                          listed ? 0 : size_t(n) * sizeof(int64_t),
-                                          listed ? 0 : size_t(n + 1) * sizeof(int64_t),
-                                          listed ? 0 : size_t(scan_temp_elems(n)) * sizeof(int64_t),
-                                          listed ? 0 : size_t(n) * sizeof(int32_t),
-                                          size_t(n) * std::min(kt, int(n_frames)) * sizeof(float),
-                                          size_t(n) * batch_tile_at(n_frames, kt, 0) * sizeof(float)})));
-  Carve cv(ctx->d_scratch);
-  if (!a.cols) {
-    int32_t* cols = cv.take<int32_t>(size_t(n));
-    RCHECK(list_columns(ctx, n, a.cp, cv, cols, &a.n_full, s));
-    a.cols = cols;
-  }
-  a.E = cv.take<float>(size_t(std::max<int64_t>(m, 1)) * n_frames);
-  a.XX = cv.take<float>(size_t(n) * n_frames);
-  double* acc = cv.take<double>(size_t(n_frames));
-  unsigned long long* next = cv.take<unsigned long long>(size_t(n_frames) * kBatchRowBlocks);
+  // E and XX, whose place the listing uses first
+  const size_t work = std::max(Carve::need({size_t(std::max<int64_t>(m, 1)) * n_frames * sizeof(float),
+                                            size_t(n) * n_frames * sizeof(float)}),
+                               listed ? size_t(0) : list_bytes(n));
   // the compact images of a tile narrower than the batch (the first tile
   // is the widest: 12 frames at kt = 64 run as 8 + 4)
-  const int widest = batch_tile_at(n_frames, kt, 0);
-  if (widest < n_frames) a.Xt = cv.take<float>(size_t(n) * widest);
+  auto images = [&](int t) {
+    const int widest = batch_tile_at(n_frames, t, 0);
+    return widest < n_frames ? size_t(n) * widest * sizeof(float) : size_t(0);
+  };
   // the back pass in row-block groups when one tile's ratios exceed L2
-  if (m > 0 && double(m) * std::min(kt, int(n_frames)) * sizeof(float) > kBatchBlockingBytes) {
+  auto partials = [&](int t) {
+    const int w = std::min(t, int(n_frames));
+    return m > 0 && double(m) * w * sizeof(float) > kBatchBlockingBytes ? size_t(n) * w * sizeof(float) : size_t(0);
+  };
+  // where the scratch cannot be had, narrower tiles, which need less
+  raptr_status got = RAPTR_OK;
+  for (;; kt /= 2) {
+    got = ctx->ensure_scratch(Carve::need({work, size_t(n_frames) * sizeof(double),
+                                           size_t(n_frames) * sizeof(unsigned long long) * kBatchRowBlocks,
+                                           listed ? size_t(0) : size_t(n) * sizeof(int32_t), sizeof(int64_t),
+                                           images(kt), partials(kt)}));
+    if (got == RAPTR_OK || kt == 4) break;
+    (void)cudaGetLastError();
+  }
+  if (got != RAPTR_OK) return got;
+  Carve cv(ctx->d_scratch);
+  unsigned char* base = cv.take<unsigned char>(work);
+  if (!listed) {
+    int32_t* cols = cv.take<int32_t>(size_t(n));
+    int64_t* n_full = cv.take<int64_t>(1);
+    RCHECK(list_columns(ctx, n, a.cp, base, cols, n_full, s));
+    a.cols = cols;
+    a.n_full = n_full;
+  }
+  Carve ex(base);
+  a.E = ex.take<float>(size_t(std::max<int64_t>(m, 1)) * n_frames);
+  a.XX = ex.take<float>(size_t(n) * n_frames);
+  double* acc = cv.take<double>(size_t(n_frames));
+  unsigned long long* next = cv.take<unsigned long long>(size_t(n_frames) * kBatchRowBlocks);
+  if (images(kt)) a.Xt = cv.take<float>(images(kt) / sizeof(float));
+  if (partials(kt)) {
     RCU(ctx->block_seg(a.cp, a.trow, m, n, s, &a.seg));
     a.seg_blocks = kBatchRowBlocks;
-    a.P = cv.take<float>(size_t(n) * std::min(kt, int(n_frames)));
+    a.P = cv.take<float>(partials(kt) / sizeof(float));
   }
   std::vector<cudaEvent_t> evs;
   if (want_times) {
