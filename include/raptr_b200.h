@@ -240,8 +240,9 @@ raptr_status raptr_sensitivity_csc(int64_t n, const int64_t* d_col_ptr, const fl
                                    float* d_s32, void* stream);
 
 typedef struct raptr_mlem_opts {
-  int32_t use_graph;   /* return when the iterations have ended (they are plain
-                        * launches: a CUDA graph of them is slower at any size) */
+  int32_t use_graph;   /* return when the iterations have ended.  They are plain
+                        * launches; a caller may capture the call itself
+                        * (use_graph 0, a first call before it) and replay it   */
   double* h_loglik;    /* optional: per-iteration Poisson log-likelihood (FP64)  */
   float* h_kernel_ms;  /* optional: 2*n_iter device times (ms) of the two passes of
                           each iteration, from CUDA events on the stream       */
@@ -370,10 +371,10 @@ raptr_status raptr_mlem_f64(raptr_ctx* ctx, int64_t m, int64_t n, const int64_t*
  * frame tile's ratios exceed ~96 MB, the back pass runs over groups of row
  * blocks of the transpose so that the ratios it gathers stay in L2.
  * n_frames must be a multiple of 4.  Each pass handles up to frame_tile
- * frames per sweep of the matrix (4, 8, 16, 32 or 64; 0 = 32): tiles of
+ * frames per sweep of the matrix (4, 8, 16, 32 or 64; 0 = 64): tiles of
  * frame_tile frames while that many remain, then the largest power of two
- * that fits (40 frames at 32: 32 + 8).  d_x and d_y must be 16-byte
- * aligned.
+ * that fits (40 frames at 32: 32 + 8); narrower ones where the scratch of
+ * these cannot be had.  d_x and d_y must be 16-byte aligned.
  * opts: with use_graph the call returns when the iterations have ended;
  * h_kernel_ms receives per iteration the forward and back-pass times. */
 raptr_status raptr_mlem_batch(raptr_ctx* ctx, int64_t m, int64_t n, int32_t n_frames, int32_t value_type,

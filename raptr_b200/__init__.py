@@ -450,8 +450,9 @@ class Context:
 
     def mlem(self, A: Matrix, y, s, x, niter: int, use_graph: bool = True, loglik: bool = False,
              kernel_times: bool = False, stream=None):
-        """MLEM iterations in place on x.  Returns the per-iteration
-        log-likelihood (loglik) and/or the (n_iter, 2) device times in ms of
+        """MLEM iterations in place on x.  With use_graph the call returns when
+        they have ended, else when they are queued on the stream (the launches
+        are the same).  Returns the per-iteration log-likelihood (loglik) and/or the (n_iter, 2) device times in ms of
         the two passes of each iteration (kernel_times), else None."""
         ll = (C.c_double * max(niter, 1))() if loglik else None
         kt = (C.c_float * max(2 * niter, 1))() if kernel_times else None
@@ -532,8 +533,9 @@ class Context:
     def mlem_batch(self, A: Matrix, Y, s, X, niter: int, frame_tile: int = 0, half: bool = True,
                    use_graph: bool = True, kernel_times: bool = False, stream=None):
         """MLEM for K frames together: Y (m, K) and X (n, K) float32,
-        row-major (frame-minor); s the one normalised sensitivity.  Returns
-        the (niter, 2) pass times with kernel_times, else None."""
+        row-major (frame-minor); s the one normalised sensitivity; use_graph
+        as in mlem().  Returns the (niter, 2) pass times with kernel_times, else
+        None."""
         K = int(X.shape[1])
         assert Y.shape == (A.m, K) and X.shape == (A.n, K) and X.is_contiguous() and Y.is_contiguous()
         vt, val, rsc, tval = self._batch_arrays(A, half)

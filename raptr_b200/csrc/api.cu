@@ -1426,10 +1426,10 @@ raptr_status mlem_impl(raptr_ctx* ctx, int64_t m, int64_t n, const MlemArrays& A
     return cudaSuccess;
   };
 
-  // Plain launches: capturing and instantiating a graph of the iterations takes
-  // 250 us and more, and its launches are no closer together (300 rows, 20
-  // iterations: 936 us with a graph, 646 without; 200,000 rows, 50 iterations:
-  // 22.6 against 22.2 ms).
+  // Plain launches: a graph of the iterations would replay up to 7 us an iteration
+  // faster (300 rows, 20 iterations: 623 us plain, 488 a replay; 57,122 rows of 70^3 3252
+  // and 3118), but capturing and instantiating it takes 250 us and more per call, so that it
+  // would pay from some 40 iterations of the smallest matrices on.
   RCU(enqueue(s));
   if (wait) RCU(cudaStreamSynchronize(s));
   if (want_times) {

@@ -4,11 +4,11 @@
 
 Builds rows [O, O+R) of the workload's system matrix (the channels in id
 order: 28,561 per angle at 70^3 x 180 angles, so O = 628342 starts at the
-23rd angle, 46 degrees), transposes it (radix sort in the channels'
-back-projection order) and runs three MLEM iterations, so that each hot
-kernel (sm_slab_kernel, rs_scatter, mlem_forward_kernel,
-mlem_back_kernel) launches a few times on a matrix larger than L2 but only
-a few GB on the device.  --build-only stops after the build.  With --forms
+23rd angle, 46 degrees), transposes it (the partition of sorted rows, in the
+channels' back-projection order) and runs three MLEM iterations, so that each
+hot kernel (sm_slab_kernel, sorted_split/copy/scatter_kernel,
+mlem_forward_kernel, mlem_back_kernel) launches a few times on a matrix larger
+than L2 but only a few GB on the device.  --build-only stops after the build.  With --forms
 it also runs the FP16 form (three iterations) and the batched form (16
 frames, two iterations).
 
