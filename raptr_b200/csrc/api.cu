@@ -1378,6 +1378,7 @@ raptr_status mlem_impl(raptr_ctx* ctx, int64_t m, int64_t n, const MlemArrays& A
     for (auto& ev : evs) RCU(cudaEventCreate(&ev));
   }
   constexpr int kAcc = 5;  // words per iteration
+  const bool drawn = rows_drawn(m, n);
   RCHECK(ctx->ensure_scratch(Carve::need({size_t(n) * sizeof(float), size_t(csc ? m : 1) * sizeof(float),
                                           size_t(kAcc) * size_t(n_iter) * sizeof(double), sizeof(double)})));
   Carve cv(ctx->d_scratch);
@@ -1404,8 +1405,9 @@ raptr_status mlem_impl(raptr_ctx* ctx, int64_t m, int64_t n, const MlemArrays& A
           err = packed ? launch_mlem_forward_packed(m, A.pseg, A.panchor, A.pword, A.rscale, d_y, d_x, rank, e, lli,
                                                     next_row, q)
                 : half ? launch_mlem_forward_half(m, d_row_ptr, d_col, A.hval, A.rscale, d_y, d_x, rank, e, lli, q,
-                                                  next_row)
-                       : launch_mlem_forward(m, d_row_ptr, d_col, d_val, d_y, d_x, rank, e, lli, q, next_row);
+                                                  drawn ? next_row : nullptr)
+                       : launch_mlem_forward(m, d_row_ptr, d_col, d_val, d_y, d_x, rank, e, lli, q,
+                                             drawn ? next_row : nullptr);
         if (want_times && err == cudaSuccess) err = cudaEventRecord(evs[size_t(3 * it + 1)], q);
         if (err == cudaSuccess)
           err = packed ? launch_mlem_back_packed(n, A.tseg, A.tanchor, A.tword, e, d_x, d_s, c, acc, true, next_col, q)

@@ -283,11 +283,15 @@ __device__ __forceinline__ int64_t warp_next(unsigned long long* next, int lane)
   return int64_t(__shfl_sync(0xffffffffu, q, 0));
 }
 
-// Below this many rows, each of which would be a draw of its own, the row passes take
-// them by a grid stride, since the draws would take longer than the rows: 57,122 rows
-// of 438 entries 73 us drawn, 51 strided; 94,000 of 724 131 and 117.  (Rows of 1535
-// entries are 1-2 % faster drawn: 57,122 155 and 158.)
-constexpr int64_t kDrawRows = int64_t(kDrawWarps) * 16;
+// Whether the FP32 and FP16 forward passes draw their m rows over n voxels, or take them
+// by a grid stride.  Below 47,360 rows (eight to a warp) the draws would take longer than
+// the rows, and up to twice as many, each a draw of its own, they do where rows are
+// short: 57,122 rows of 40^3 (438 entries) 73 us drawn, 51 strided; 94,000 of 70^3 (724) 131
+// and 117; but of 100^3 (1535 entries) 57,122 155 and 158, 90,000 231 and 236.
+inline bool rows_drawn(int64_t m, int64_t n) {
+  const int64_t one = int64_t(kDrawWarps) * 8;
+  return m >= 2 * one || (m >= one && n >= 600000);
+}
 
 // Rows a draw takes: 16 (one draw per row makes the forward pass of 5.14M rows
 // twice as slow, one per 16 takes 7 % off the grid stride's time), fewer where

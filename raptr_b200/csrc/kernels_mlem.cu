@@ -787,7 +787,6 @@ cudaError_t launch_mlem_forward(int64_t m, const int64_t* rp, const int32_t* col
                                 const float* x, const int32_t* rank, float* e, double* d_ll, cudaStream_t s,
                                 unsigned long long* next) {
   if (m > 0) {
-    if (m < kDrawRows) next = nullptr;
     mlem_forward_kernel<<<row_grid(m), kThreads, 0, s>>>(m, rp, col, val, y, x, rank, e, d_ll, next);
     note_launches(1);
   }

@@ -642,7 +642,6 @@ cudaError_t launch_mlem_forward_half(int64_t m, const int64_t* rp, const int32_t
                                      const float* rscale, const float* y, const float* x, const int32_t* rank,
                                      float* e, double* d_ll, cudaStream_t s, unsigned long long* next) {
   if (m <= 0) return cudaSuccess;
-  if (m < kDrawRows) next = nullptr;
   mlem_forward_half_kernel<<<grid_rows(m), kThreads, 0, s>>>(m, rp, col, hval, rscale, y, x, rank, e, d_ll, next);
   note_launches(1);
   return cudaGetLastError();

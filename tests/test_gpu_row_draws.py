@@ -17,12 +17,14 @@ WARPS = 148 * 40
 RTOL = 170 * 2.0 ** -24
 
 
-@pytest.mark.parametrize("m", [WARPS * 16 - 1, WARPS * 16, WARPS * 128 - 1, WARPS * 128, WARPS * 128 + 7])
-def test_row_draws(rlib, m):
+# (rows over 600,000 voxels and more are drawn from half as many on)
+@pytest.mark.parametrize("m,n", [(WARPS * 16 - 1, 500), (WARPS * 16, 500), (WARPS * 128 - 1, 500), (WARPS * 128, 500),
+                                 (WARPS * 128 + 7, 500), (WARPS * 8 - 1, 600000), (WARPS * 8, 600000),
+                                 (WARPS * 8, 599999)])
+def test_row_draws(rlib, m, n):
     import torch
 
     rng = np.random.default_rng(m)
-    n = 500
     lens = rng.integers(1, 4, m)
     rp = np.r_[0, np.cumsum(lens)].astype(np.int64)
     row = np.repeat(np.arange(m), lens)
